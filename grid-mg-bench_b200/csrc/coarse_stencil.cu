@@ -1,4 +1,4 @@
-// coarse_stencil.cu -- 9-point coarse Dirac stencil on CUDA cores (FP64 / FP32).
+// coarse_stencil.cu -- 9-point coarse Dirac stencil in FP64 and FP32.
 //
 // Restates CoarsenedMatrix::M / Mdag / MdirCalc / Mdiag
 // (include/CoarsenedMatrixUpstream.h:546-742) and the multi-RHS form
@@ -8,16 +8,18 @@
 //
 // with Mdag = G5C M G5C (sign flip of the upper half of the basis index on
 // load and store, no temporary).  The reference runs one thread per (site,
-// row) and re-reads every link element once per RHS; here one CTA owns a
-// site, stages A_p(x) and the neighbour's R x N tile in shared memory
-// (transposed so that the basis index is the contiguous one), and every
-// thread accumulates a TR x TB register tile of (rhs, row) outputs, so a link
-// element is read from HBM once for all R right-hand sides.
+// row) and re-reads every link element once per RHS; here a link element is
+// read from HBM once for all R right-hand sides.  Three forms:
+// coarse_mma_kernel (FP64 tensor cores, most sizes of both precisions),
+// coarse_simt_pipe_kernel (FP32 pipe, FP32 fields with many right-hand sides)
+// and the single-RHS kernels (small lattices).
 //
 // Links are kept site-major, [V][9][N][N], so that one site's 9 matrices are
 // one contiguous stream.
 #include <algorithm>
+#include <type_traits>
 
+#include "f64_mma.cuh"
 #include "gmg_internal.cuh"
 
 namespace gmg {
@@ -102,93 +104,244 @@ template <class C> __device__ __forceinline__ C cconj(C a) {
   return a;
 }
 
-template <class T, int TR, int TB>
-__global__ void __launch_bounds__(256) coarse_simt_kernel(
-    const typename cplx_t<T>::type* __restrict__ links, int link_pts, int pbase, const int32_t* __restrict__ site_map,
-    const int32_t* __restrict__ nbr, int dag,
-    const typename cplx_t<T>::type* __restrict__ in, typename cplx_t<T>::type* __restrict__ out,
-    int V, int N, int nrhs, const int32_t* __restrict__ active, int R, int p0, int p1, int g5) {
+// ---------------------------------------------------------------------------
+// The stencil on the FP64 tensor cores (f64_mma.cuh), for FP64 fields and for
+// FP32 ones widened on load.  A unit is one site, 8 MT rows and 4 RQ right-hand
+// sides; a warp forms a unit's sum over its share of the site's (point, basis)
+// contraction with the next step's operands requested one step ahead, KS warps
+// of the CTA taking the points in turn ranges and adding their tiles through
+// shared memory in a fixed order.
+// What bounds it: the MMA rate (the links are used once per R right-hand
+// sides, 8 N N R flops per 16 N N bytes: above about 10 FP64 right-hand sides
+// the arithmetic takes longer than the links).  The register-tiled CUDA-core
+// kernels before it were bound by their shared-memory operand reads and one
+// barrier pair per point.  At 8^4, nbasis 32, 32 RHS, FP64: 536 -> 356 us
+// (27 TFLOP/s of the 37 the MMAs reach; two register sets leave 10 warps per SM,
+// which do not always cover the links' DRAM latency); 4096 sites, nbasis 40, 7
+// RHS: 1276 -> 197 us; 840 sites, nbasis 40, 5 RHS, FP32: 284 -> 41 us.
+// sel (nullable): the output sites (gridDim.x of them) instead of all; skip
+// (nullable): per site, bit p leaves point p out.
+// ---------------------------------------------------------------------------
+template <class C> struct MmaArgs {
+  const C* links;
+  int link_pts, pbase;
+  const int32_t* site_map;
+  const int32_t* nbr;
+  int dag;
+  const C* in;
+  C* out;
+  int V, N, nrhs;
+  const int32_t* active;
+  int R, p0, p1, g5;
+  const int32_t* sel;
+  const uint8_t* skip;
+  int units, rchunks, G, KS;  // units per site (rchunks per row chunk), units and point shares per CTA
+};
+
+// threads of a CTA: 9 warps (a stencil's points) where the tile leaves the
+// registers for three warps on a scheduler, else 8
+constexpr int mma_threads(int tiles) { return tiles <= 8 ? 288 : 256; }
+
+
+template <class T, int MT, int RQ>
+__global__ void __launch_bounds__(mma_threads(MT * RQ)) coarse_mma_kernel(const MmaArgs<typename cplx_t<T>::type> a) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* AT = reinterpret_cast<C*>(smem_raw);  // [N][N]   AT[bb][b] = A[b][bb]
-  C* XT = AT + N * N;                      // [N][R]   XT[bb][r] = in(nbr, r)[bb]
-  const int NBT = (N + TB - 1) / TB;
-  const int NRT = (R + TR - 1) / TR;
-  const int ntiles = NBT * NRT;
-  const int t = threadIdx.x;
-  const int bt = t % NBT, rt = t / NBT;
-  const int half = N / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int N = a.N, ks = warp % a.KS, g = warp / a.KS, u = blockIdx.y * a.G + g;
+  const int site = a.sel ? a.sel[blockIdx.x] : (int)blockIdx.x;
+  const int mc = u / a.rchunks, rc = u - mc * a.rchunks;
+  const int kk = lane & 3, part = (lane >> 2) & 1, half = N / 2;
+  double acc[MT][RQ][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int q = 0; q < RQ; ++q) acc[m][q][0] = acc[m][q][1] = 0.0;
 
-  for (int site = blockIdx.x; site < V; site += gridDim.x) {
-    const int64_t lsite = site_map ? site_map[site] : site;
-    C acc[TR][TB];
+  if (u < a.units) {
+    // rows and right-hand sides past the end repeat the last one; their results are not stored
+    const int sb = a.dag ? 1 : N, sk = a.dag ? N : 1;
+    int rowoff[MT], foff[RQ];
 #pragma unroll
-    for (int j = 0; j < TR; ++j)
+    for (int m = 0; m < MT; ++m) rowoff[m] = min((mc * MT + m) * 8 + (lane >> 2), N - 1) * sb;
 #pragma unroll
-      for (int i = 0; i < TB; ++i) acc[j][i] = C{0, 0};
-
-    for (int p = p0; p < p1; ++p) {
-      const C* Ap = links + (lsite * link_pts + (p - pbase)) * N * N;
-      const int nb = nbr ? nbr[(int64_t)p * V + site] : site;
-      __syncthreads();
-      if (dag) {  // AT[bb][b] = (A^dag)[b][bb] = conj(A[bb][b])
-        for (int k = t; k < N * N; k += blockDim.x) AT[k] = cconj(Ap[k]);
-      } else {
-        for (int k = t; k < N * N; k += blockDim.x) {
-          const int b = k / N, bb = k % N;
-          AT[bb * N + b] = Ap[k];
+    for (int q = 0; q < RQ; ++q) {
+      const int r = min((rc * RQ + q) * 4 + (lane >> 3), a.R - 1);
+      foff[q] = (a.active ? a.active[r] : r) * N;
+    }
+    const uint32_t s1 = f64mma::second_sign(part, a.dag != 0);
+    const int64_t lsite = a.site_map ? a.site_map[site] : site;
+    const C* lp = a.links + (lsite * a.link_pts - a.pbase) * (int64_t)N * N;
+    const int mynb = (a.nbr && lane < 9) ? a.nbr[(int64_t)lane * a.V + site] : site;
+    const int npts = a.p1 - a.p0;
+    unsigned pts = ((1u << (a.p0 + (ks + 1) * npts / a.KS)) - 1) & ~((1u << (a.p0 + ks * npts / a.KS)) - 1);
+    if (a.skip) pts &= ~(unsigned)a.skip[site];
+    // Both operands are requested two steps ahead of their use, into the other
+    // of two register sets.
+    if (pts) {
+      C av[2][MT], fv[2][RQ];
+      int k4 = 0, left = __popc(pts) * ((N + 3) / 4), k0 = 0;
+      const C *Ap, *xp;
+      auto at_point = [&]() {
+        const int p = __ffs(pts) - 1;
+        Ap = lp + (int64_t)p * N * N;
+        xp = a.in + (int64_t)__shfl_sync(0xffffffffu, mynb, p) * a.nrhs * N;
+      };
+      auto request = [&](C (&A)[MT], C (&F)[RQ]) {
+        const int k = k4 + kk;
+        const bool in_k = k < N;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) A[m] = in_k ? __ldg(Ap + rowoff[m] + k * sk) : C{0, 0};
+#pragma unroll
+        for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(xp + foff[q] + k) : C{0, 0};
+        k4 += 4;
+        if (k4 >= N) {
+          k4 = 0;
+          pts &= pts - 1;
+          if (pts) at_point();
         }
-      }
-      for (int k = t; k < R * N; k += blockDim.x) {
-        const int r = k / N, bb = k % N;
-        const int slot = active ? active[r] : r;
-        C v = in[((int64_t)nb * nrhs + slot) * N + bb];
-        if (g5 && bb >= half) { v.x = -v.x; v.y = -v.y; }
-        XT[bb * R + r] = v;
-      }
-      __syncthreads();
-      if (t < ntiles) {
-        for (int bb = 0; bb < N; ++bb) {
-          C a[TB], x[TR];
+      };
+      auto multiply = [&](const C (&A)[MT], const C (&F)[RQ]) {
+        const uint32_t g5 = (a.g5 && k0 + kk >= half) ? 0x80000000u : 0u;
+        double b0[RQ], b1[RQ];
 #pragma unroll
-          for (int i = 0; i < TB; ++i) {
-            const int b = bt * TB + i;
-            a[i] = b < N ? AT[bb * N + b] : C{0, 0};
-          }
+        for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, g5, s1 ^ g5, b0[q], b1[q]);
 #pragma unroll
-          for (int j = 0; j < TR; ++j) {
-            const int r = rt * TR + j;
-            x[j] = r < R ? XT[bb * R + r] : C{0, 0};
-          }
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
-          for (int j = 0; j < TR; ++j)
+          for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].x, b0[q]);
 #pragma unroll
-            for (int i = 0; i < TB; ++i) acc[j][i] = cmul_add(acc[j][i], a[i], x[j]);
-        }
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+          for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].y, b1[q]);
+        k0 = k0 + 4 >= N ? 0 : k0 + 4;
+      };
+      at_point();
+      request(av[0], fv[0]);
+      for (;;) {
+        if (left > 1) request(av[1], fv[1]);
+        multiply(av[0], fv[0]);
+        if (--left == 0) break;
+        if (left > 1) request(av[0], fv[0]);
+        multiply(av[1], fv[1]);
+        if (--left == 0) break;
       }
     }
-    if (t < ntiles) {
+  }
+
+  auto store = [&](int m, int q, double re, double im) {
+    const int b = (mc * MT + m) * 8 + (lane >> 2), r = (rc * RQ + q) * 4 + kk;
+    if (b >= N || r >= a.R) return;
+    if (a.g5 && b >= half) {
+      re = -re;
+      im = -im;
+    }
+    const int slot = a.active ? a.active[r] : r;
+    C v;
+    v.x = re;
+    v.y = im;
+    a.out[((int64_t)site * a.nrhs + slot) * N + b] = v;
+  };
+  if (a.KS == 1) {
+    if (u < a.units) {
 #pragma unroll
-      for (int j = 0; j < TR; ++j) {
-        const int r = rt * TR + j;
-        if (r >= R) continue;
-        const int slot = active ? active[r] : r;
-        C* o = out + ((int64_t)site * nrhs + slot) * N;
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int i = 0; i < TB; ++i) {
-          const int b = bt * TB + i;
-          if (b >= N) continue;
-          C v = acc[j][i];
-          if (g5 && b >= half) { v.x = -v.x; v.y = -v.y; }
-          o[b] = v;
-        }
+        for (int q = 0; q < RQ; ++q) store(m, q, acc[m][q][0], acc[m][q][1]);
+    }
+    return;
+  }
+  double2* red = reinterpret_cast<double2*>(smem_raw) + (int64_t)g * a.KS * MT * RQ * 32;
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int q = 0; q < RQ; ++q)
+      red[(ks * MT * RQ + m * RQ + q) * 32 + lane] = make_double2(acc[m][q][0], acc[m][q][1]);
+  __syncthreads();
+  if (u < a.units) {
+    for (int t = ks; t < MT * RQ; t += a.KS) {
+      double re = 0.0, im = 0.0;
+      for (int j = 0; j < a.KS; ++j) {
+        const double2 v = red[(j * MT * RQ + t) * 32 + lane];
+        re += v.x;
+        im += v.y;
       }
+      store(t / RQ, t % RQ, re, im);
     }
   }
 }
 
+template <class T, int MT, int RQ>
+static gmg_status launch_mma(const MmaArgs<typename cplx_t<T>::type>& a, int nsites, cudaStream_t s) {
+  auto kern = coarse_mma_kernel<T, MT, RQ>;
+  const size_t smem = a.KS == 1 ? 0 : sizeof(double2) * 32 * MT * RQ * (size_t)a.G * a.KS;
+  if (smem > 48 * 1024)
+    GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  KernelTimer kt("coarse_simt", s);
+  kern<<<dim3(nsites, (a.units + a.G - 1) / a.G), 32 * a.G * a.KS, smem, s>>>(a);
+  GMG_CUDA(cudaGetLastError());
+  return GMG_OK;
+}
+
+// Launch shape: quads of right-hand sides per unit (w, in `chunks` chunks),
+// units (G) and point shares (KS) per CTA.  w gives the fewest padded quads
+// (each chunk reads the links once more, counted as half a quad).  One warp per
+// unit is fastest where the lattice fills the chip (4096 sites, nbasis 32, 32 RHS, FP64:
+// 356 us, 431 with two shares); below that the points are split until
+// every SM has about 12 warps, or 24 of the small tiles, whose steps are too
+// short to hide the operands' latency (840 sites, nbasis 40, 5 RHS, FP32: 39 us
+// with 5 shares, 44 with 2, 48 with 1).
+struct MmaShape {
+  int w, chunks, G, KS;
+};
+static MmaShape mma_shape(int64_t nsites, int npts, int MT, int mchunks, int rq) {
+  MmaShape sh{1, rq, 1, 1};
+  for (int w = 2; w <= 4; ++w) {
+    const int u = (rq + w - 1) / w;
+    if (u * (2 * w + 1) <= sh.chunks * (2 * sh.w + 1)) sh = MmaShape{w, u, 1, 1};
+  }
+  const int units = mchunks * sh.chunks, maxw = mma_threads(MT * sh.w) / 32;
+  const int64_t want = 148 * (MT * sh.w > 10 ? 12 : 24);
+  for (const int ks : {1, 2, 3, 5, 9}) {
+    sh.KS = std::min(ks, std::min(npts, maxw));
+    if (nsites * units * sh.KS >= want) break;
+  }
+  sh.G = std::min(units, maxw / sh.KS);
+  return sh;
+}
+
+template <class T>
+static gmg_status coarse_mma(const LinkSel& L, const void* in, void* out, int V, int N, int nrhs,
+                             const int32_t* active, int R, int p0, int p1, int g5, const int32_t* sel, int nsel,
+                             const uint8_t* skip, cudaStream_t s) {
+  typedef typename cplx_t<T>::type C;
+  const int mt = (N + 7) / 8, mchunks = (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
+  const int nsites = sel ? nsel : V, npts = p1 - p0;
+  if (nsites == 0) return GMG_OK;
+  const MmaShape sh = mma_shape(nsites, npts, MT, mchunks, (R + 3) / 4);
+  MmaArgs<C> a{reinterpret_cast<const C*>(L.links), L.link_pts, L.pbase, L.site_map, L.nbr, L.dag,
+               reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), V, N, nrhs, active, R, p0, p1, g5,
+               sel, skip, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
+  auto by_rq = [&](auto mtc) -> gmg_status {
+    constexpr int M = decltype(mtc)::value;
+    switch (sh.w) {
+      case 1: return launch_mma<T, M, 1>(a, nsites, s);
+      case 2: return launch_mma<T, M, 2>(a, nsites, s);
+      case 3: return launch_mma<T, M, 3>(a, nsites, s);
+      default: return launch_mma<T, M, 4>(a, nsites, s);
+    }
+  };
+  switch (MT) {
+    case 1: return by_rq(std::integral_constant<int, 1>());
+    case 2: return by_rq(std::integral_constant<int, 2>());
+    case 3: return by_rq(std::integral_constant<int, 3>());
+    case 4: return by_rq(std::integral_constant<int, 4>());
+    default: return by_rq(std::integral_constant<int, 5>());
+  }
+}
+
 // ---------------------------------------------------------------------------
-// The multi-RHS stencil on the CUDA cores, pipelined: a CTA walks the (site,
+// The multi-RHS FP32 stencil on the CUDA cores, pipelined: a CTA walks the (site,
 // point) items of its sites; while it multiplies item k, the link matrix and
 // the neighbour's R vectors of item k + 1 are copied into the other half of
 // its shared memory with cp.async.  A thread owns a TR x TB tile of the R x N
@@ -338,8 +491,7 @@ static bool launch_simt_pipe(const LinkSel& L, const void* in, void* out, int V,
   typedef typename cplx_t<T>::type C;
   if (N % TB || R % TR || (N / TB) * (R / TR) > 256 || p1 <= p0) return false;
   const size_t smem = sizeof(C) * 2 * (size_t)(N + R) * (N + 1);
-  // at least 3 CTAs per SM: with two (FP64 nbasis 40 x 40 RHS, the coarse-of-
-  // coarse construction) the kernel without the pipeline, at 4, was faster
+  // at least 3 CTAs per SM
   if (smem > 72 * 1024) return false;
   const int threads = std::max(32, ((N / TB) * (R / TR) + 31) / 32 * 32);
   auto kern = N == 32 ? coarse_simt_pipe_kernel<T, TR, TB, 32>
@@ -363,31 +515,6 @@ static bool launch_simt_pipe(const LinkSel& L, const void* in, void* out, int V,
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) *st = fail(GMG_ERR_CUDA, std::string("coarse apply: ") + cudaGetErrorString(e));
   return true;
-}
-
-template <class T, int TR, int TB>
-static gmg_status launch_simt(const LinkSel& L, const void* in, void* out,
-                              int V, int N, int nrhs, const int32_t* active, int R, int p0, int p1,
-                              int g5, cudaStream_t s) {
-  typedef typename cplx_t<T>::type C;
-  const int ntiles = ((N + TB - 1) / TB) * ((R + TR - 1) / TR);
-  GMG_CHECK(ntiles <= 256, GMG_ERR_UNSUPPORTED, "coarse apply: nbasis x nrhs tile too large");
-  const int threads = std::max(32, (ntiles + 31) / 32 * 32);
-  const size_t smem = sizeof(C) * ((size_t)N * N + (size_t)N * R);
-  GMG_CHECK(smem <= 227 * 1024, GMG_ERR_UNSUPPORTED, "coarse apply: shared-memory tile too large");
-  auto kern = coarse_simt_kernel<T, TR, TB>;
-  GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int dev = 0, nsm = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-  const int grid = std::min(V, nsm * std::max(per_sm, 1) * 4);
-  KernelTimer kt("coarse_simt", s);
-  kern<<<grid, threads, smem, s>>>(reinterpret_cast<const C*>(L.links), L.link_pts, L.pbase, L.site_map, L.nbr, L.dag,
-                                   reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), V, N,
-                                   nrhs, active, R, p0, p1, g5);
-  GMG_CUDA(cudaGetLastError());
-  return GMG_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -570,19 +697,31 @@ gmg_status coarse_apply_simt_ex(gmg_coarse* h, int src, int V, const int32_t* si
     return fail(GMG_ERR_UNSUPPORTED, "coarse apply: unsupported compute precision for SIMT path");
   }
   GMG_CHECK(L.links != nullptr, GMG_ERR_STATE, "coarse apply: link source not built");
-  if (R == 1 && !active && N <= 64) {
+  // One right-hand side: the CUDA-core kernels where a site's links fit their
+  // staging buffer (nbasis 24 in FP64, 32 in FP32) and the lattice is small
+  // enough to be bound by latency.  FP64 us, CUDA cores / tensor cores: 256
+  // sites, nbasis 24: 6.2 / 6.3, nbasis 32: 14 / 10; 768 sites, nbasis 24: 14.4 /
+  // 12.3; 4096 sites, nbasis 8: 10.3 / 12.3, nbasis 32: 161 / 98.  FP32: 1024
+  // sites, nbasis 32: 16 / 20, nbasis 40: 45 / 31; 4096, nbasis 24: 44 / 38.
+  const int64_t vnn = (int64_t)V * N * N;
+  if (R == 1 && !active &&
+      (compute == GMG_F64 ? N <= 24 && vnn < 768 * 24 * 24 : N <= 32 && vnn < 4096 * 24 * 24)) {
     if (compute == GMG_F64) return launch_1rhs<double>(L, in, out, V, N, nrhs, 0, p0, p1, g5, s);
     return launch_1rhs<float>(L, in, out, V, N, nrhs, 0, p0, p1, g5, s);
   }
+  // the sizes the apply takes
+  const size_t esz = compute == GMG_F64 ? sizeof(double2) : sizeof(float2);
+  GMG_CHECK(R < 4 || ((N + 3) / 4) * ((R + 3) / 4) <= 256, GMG_ERR_UNSUPPORTED,
+            "coarse apply: nbasis x nrhs tile too large");
+  GMG_CHECK(esz * N * (size_t)(N + R) <= 227 * 1024, GMG_ERR_UNSUPPORTED, "coarse apply: nbasis x nrhs too large");
+  if (compute == GMG_F64) return coarse_mma<double>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, nullptr, 0, nullptr, s);
+  // FP32 with 28 right-hand sides or more at nbasis 32 to 40, in whole 4 x 4
+  // tiles: the FP32 pipe's twice higher rate still wins there (768 sites, nbasis
+  // 32, 32 RHS: 65 us against 83 on the FP64 tensor cores; 24 RHS: 64 against 62;
+  // nbasis 24, 32 RHS: 52 against 50; nbasis 48: 224 against 168)
   gmg_status st = GMG_OK;
-  if (compute == GMG_F64) {
-    if (R >= 4 && launch_simt_pipe<double, 4, 2>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s, &st)) return st;
-    if (R >= 4) return launch_simt<double, 4, 4>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s);
-    return launch_simt<double, 1, 2>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s);
-  }
-  if (R >= 4 && launch_simt_pipe<float, 4, 4>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s, &st)) return st;
-  if (R >= 4) return launch_simt<float, 4, 4>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s);
-  return launch_simt<float, 1, 2>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s);
+  if (R >= 28 && N >= 32 && N <= 40 && launch_simt_pipe<float, 4, 4>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, s, &st)) return st;
+  return coarse_mma<float>(L, in, out, V, N, nrhs, active, R, p0, p1, g5, nullptr, 0, nullptr, s);
 }
 
 gmg_status coarse_apply_simt(gmg_coarse* h, int p0, int p1, bool g5, int compute, int vec_prec,

@@ -1,0 +1,73 @@
+"""FP64 tensor-core forms (complex products by mma.sync m8n8k4) against the FP64 oracle.
+
+Sizes at the edges of the kernels' tiles: 8 rows, 4 right-hand sides, 4
+contracted complex numbers, up to 5 row tiles and 4 right-hand-side quads per
+warp.  FP64 results differ from the oracle's by the order of their sums only
+(1e-15 relative squared deviation); FP32 fields are widened on load and rounded
+once on store (1e-7, as the other FP32 tests).
+"""
+import numpy as np
+import pytest
+import torch
+
+import gmg
+import inputs
+import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TOL = {torch.complex128: 1e-15, torch.complex64: 1e-7}
+
+
+def _dev(a, dt):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda().to(dt)
+
+
+def _host(t):
+    return t.cpu().numpy().astype(np.complex128)
+
+
+@pytest.mark.parametrize("dt", [torch.complex128, torch.complex64])
+@pytest.mark.parametrize("dims,N,R", [
+    ((2, 2, 2, 2), 2, 2),      # one partial tile in every direction
+    ((3, 2, 5, 2), 8, 4),      # exactly one tile
+    ((4, 3, 2, 3), 10, 17),    # remainders of rows, of k and of the quads; 5 quads in chunks
+    ((2, 2, 2, 3), 40, 5),     # five row tiles
+    ((2, 1, 2, 2), 42, 16),    # six row tiles: two row chunks
+    ((2, 2, 2, 2), 66, 3),     # nine row tiles
+    ((8, 6, 8, 8), 26, 1),     # one right-hand side on a large lattice
+    ((8, 8, 6, 8), 12, 13),    # one warp per unit (no split over points)
+])
+@pytest.mark.parametrize("op", ["M", "Mdag", "Mdiag"])
+def test_stencil(dims, N, R, dt, op):
+    r = inputs.rng(stream=700 + N + R)
+    V = int(np.prod(dims))
+    A = inputs.random_links(dims, N, r)
+    x = inputs.gaussian_field((V, R, N), r)
+    cm = gmg.CoarsenedMatrix(dims, N)
+    cm.set_links(A)
+    cm.prepare("f32")
+    ref = orc.coarse_apply(dims, A, x, {"M": orc.OP_M, "Mdag": orc.OP_MDAG, "Mdiag": orc.OP_MDIAG}[op])
+    inp = _dev(x, dt)
+    out = torch.full_like(inp, float("nan"))  # every entry is written
+    getattr(cm, op)(inp, out)
+    assert orc.rel_dev_sq(ref, _host(out)) < TOL[dt]
+
+
+def test_stencil_active_list():
+    dims, N = (4, 2, 3, 2), 18
+    r = inputs.rng(stream=790)
+    A = inputs.random_links(dims, N, r)
+    x = inputs.gaussian_field((48, 9, N), r)
+    cm = gmg.CoarsenedMatrix(dims, N)
+    cm.set_links(A)
+    inp = _dev(x, torch.complex128)
+    out = torch.full_like(inp, 7.0)
+    active = [8, 0, 3, 5, 1]
+    cm.Mdag(inp, out, active=active)
+    ref, got = orc.coarse_apply(dims, A, x, orc.OP_MDAG), _host(out)
+    for q in range(9):
+        if q in active:
+            assert orc.rel_dev_sq(ref[:, q], got[:, q]) < 1e-15
+        else:
+            assert np.all(got[:, q] == 7.0)
