@@ -336,7 +336,7 @@ gmg_status gmg_agg_project(gmg_agg* h, gmg_prec compute, gmg_prec vec_prec, int 
   GMG_CHECK(h->basis_set, GMG_ERR_STATE, "gmg_agg_project: basis not set");
   GMG_CHECK(nrhs >= 1 && nrhs <= 64, GMG_ERR_ARGUMENT, "gmg_agg_project: nrhs must be in [1, 64]");
   GMG_CHECK(vec_prec_ok(vec_prec), GMG_ERR_ARGUMENT, "gmg_agg_project: vectors must be F64 or F32");
-  return agg_project(h, compute, vec_prec, nrhs, fine, coarse, nullptr, S(s));
+  return agg_project(h, compute, vec_prec, nrhs, fine, coarse, S(s));
 }
 
 gmg_status gmg_agg_promote(gmg_agg* h, gmg_prec compute, gmg_prec vec_prec, int nrhs, const void* coarse,

@@ -1,4 +1,4 @@
-// block_ops.cu -- block projection, promotion and orthonormalisation (CUDA cores).
+// block_ops.cu -- block projection and promotion in FP64 and FP32.
 //
 // Restates blockLutedInnerProduct / blockLutedAxpy / blockLutedOrthonormalise
 // (include/CoarsenedMatrixUpstreamImprovedDirsaveLut.h:70-240, multi-RHS form
@@ -13,8 +13,9 @@
 // so one block's N x K panel is contiguous.  Fine fields stay in the caller's
 // [site][rhs][dof] layout and are gathered through blk_sites[c][sb].
 #include <algorithm>
-#include <cmath>
+#include <type_traits>
 
+#include "f64_mma.cuh"
 #include "gmg_internal.cuh"
 
 namespace gmg {
@@ -22,29 +23,6 @@ namespace gmg {
 template <class T> struct ctype;
 template <> struct ctype<double> { typedef double2 t; };
 template <> struct ctype<float> { typedef float2 t; };
-
-template <class Cx> __device__ __forceinline__ Cx cfma(Cx acc, Cx a, Cx b) {
-  acc.x = fma(a.x, b.x, acc.x);
-  acc.x = fma(-a.y, b.y, acc.x);
-  acc.y = fma(a.x, b.y, acc.y);
-  acc.y = fma(a.y, b.x, acc.y);
-  return acc;
-}
-// acc += conj(a) b
-template <class Cx> __device__ __forceinline__ Cx cfma_conj(Cx acc, Cx a, Cx b) {
-  acc.x = fma(a.x, b.x, acc.x);
-  acc.x = fma(a.y, b.y, acc.x);
-  acc.y = fma(a.x, b.y, acc.y);
-  acc.y = fma(-a.y, b.x, acc.y);
-  return acc;
-}
-
-static int num_sms() {
-  int dev = 0, n = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
-}
 
 // ---------------------------------------------------------------------------
 // tables and basis layout
@@ -137,427 +115,424 @@ gmg_status agg_prepare_f32(gmg_agg* h, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// project: coarse[c][r][i] = sum_k conj(V[c][i][k]) F[site(c,k)][r][k % dof]
-// CTA per block; K chunked by KS sites; TR x TB register tiles over (rhs, i).
-// `mask` (nullable, int8 per fine site) restricts the sum to a face / parity
-// subset as the masked LUTs of CoarsenOperator do (...DirsaveLut.h:985-1005).
-// ---------------------------------------------------------------------------
-// `sel` (nullable, nsel entries): the in-block site indices the sum runs over,
+// project: out[c][r][i] = sum_k conj(V[c][i][k]) F[site(c,k)][r][k % dof]
+// on the FP64 tensor cores (f64_mma.cuh), FP64 fields and FP32 ones widened on
+// load.  CTA per block; a unit is 8 MT basis vectors and 4 RQ right-hand sides,
+// a warp sums the unit over the block's sites ks, ks + KS, ... with the operands
+// of the next step requested one step ahead, and the KS warps of a unit add
+// their tiles through shared memory in a fixed order.
+// What bounds it: the MMA rate (8 N R flops per 16 (N + R) bytes: above about 8
+// right-hand sides the arithmetic takes longer than the reads).  The register-
+// tiled CUDA-core kernels before it were bound by shared-memory operand reads
+// and staging.  32^4, nbasis 32, 32 RHS, 4^4 blocks, FP64:
+// 7.27 -> 3.69 ms (28 TFLOP/s of 37); 16^4, nbasis 24, 12 RHS: 534 -> 95 us, in
+// FP32 2428 -> 84 us.
+// sel (nullable, nsel entries): the in-block site indices the sum runs over,
 // the same for every block (a face of the block); without it all bv sites.
-template <class T, int TR, int TB, int KS>
-__global__ void __launch_bounds__(256) project_kernel(
-    const typename ctype<T>::t* __restrict__ basis, const int32_t* __restrict__ blk_sites,
-    const typename ctype<T>::t* __restrict__ fine, typename ctype<T>::t* __restrict__ coarse,
-    int Vc, int N, int dof, int bv, int nrhs, const int8_t* __restrict__ mask, int accumulate,
-    const int32_t* __restrict__ sel, int nsel) {
+// The result goes to out[c * cstr + r * rstr + i * istr].
+// ---------------------------------------------------------------------------
+template <class Cx> struct ProjArgs {
+  const Cx* basis;
+  const int32_t* blk_sites;
+  const Cx* fine;
+  Cx* out;
+  int64_t cstr, rstr, istr;
+  int N, dof, bv, nrhs;
+  const int32_t* sel;
+  int nsel;
+  int units, rchunks, G, KS;
+};
+
+constexpr int kProjWarps = 8;
+
+template <class T, int MT, int RQ>
+__global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const ProjArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int KC = KS * dof;
-  Cx* VT = reinterpret_cast<Cx*>(smem_raw);  // [KC][N]
-  Cx* FT = VT + KC * N;                       // [KC][R]
-  const int R = nrhs;
-  const int NBT = (N + TB - 1) / TB, NRT = (R + TR - 1) / TR;
-  const int ntiles = NBT * NRT;
-  const int t = threadIdx.x, bt = t % NBT, rt = t / NBT;
-  const int64_t K = (int64_t)bv * dof;
-  for (int c = blockIdx.x; c < Vc; c += gridDim.x) {
-    Cx acc[TR][TB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int N = a.N, dof = a.dof, ks = warp % a.KS, g = warp / a.KS, u = blockIdx.y * a.G + g;
+  const int mc = u / a.rchunks, rc = u - mc * a.rchunks;
+  const int kk = lane & 3, part = (lane >> 2) & 1;
+  const int64_t c = blockIdx.x, K = (int64_t)a.bv * dof;
+  const int nsites = a.sel ? a.nsel : a.bv;
+  double acc[MT][RQ][2];
 #pragma unroll
-    for (int j = 0; j < TR; ++j)
+  for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int i = 0; i < TB; ++i) acc[j][i] = Cx{0, 0};
-    const Cx* Vb = basis + (int64_t)c * N * K;
-    const int nsites = sel ? nsel : bv;
-    for (int sb0 = 0; sb0 < nsites; sb0 += KS) {
-      const int ns = min(KS, nsites - sb0);
-      const int kc = ns * dof;
-      __syncthreads();
-      for (int e = t; e < N * kc; e += blockDim.x) {
-        const int i = e / kc, kk = e % kc;
-        const int sl = kk / dof, a = kk % dof;
-        const int sb = sel ? sel[sb0 + sl] : sb0 + sl;
-        VT[kk * N + i] = Vb[(int64_t)i * K + (int64_t)sb * dof + a];
-      }
-      for (int e = t; e < ns * R * dof; e += blockDim.x) {
-        const int sl = e / (R * dof), rem = e % (R * dof);
-        const int r = rem / dof, a = rem % dof;
-        const int sf = blk_sites[(int64_t)c * bv + (sel ? sel[sb0 + sl] : sb0 + sl)];
-        Cx v = fine[((int64_t)sf * nrhs + r) * dof + a];
-        if (mask && !mask[sf]) v = Cx{0, 0};
-        FT[(sl * dof + a) * R + r] = v;
-      }
-      __syncthreads();
-      if (t < ntiles) {
-        for (int kk = 0; kk < kc; ++kk) {
-          Cx a[TB], x[TR];
-#pragma unroll
-          for (int i = 0; i < TB; ++i) {
-            const int ii = bt * TB + i;
-            a[i] = ii < N ? VT[kk * N + ii] : Cx{0, 0};
-          }
-#pragma unroll
-          for (int j = 0; j < TR; ++j) {
-            const int r = rt * TR + j;
-            x[j] = r < R ? FT[kk * R + r] : Cx{0, 0};
-          }
-#pragma unroll
-          for (int j = 0; j < TR; ++j)
-#pragma unroll
-            for (int i = 0; i < TB; ++i) acc[j][i] = cfma_conj(acc[j][i], a[i], x[j]);
-        }
-      }
-    }
-    if (t < ntiles) {
-#pragma unroll
-      for (int j = 0; j < TR; ++j) {
-        const int r = rt * TR + j;
-        if (r >= R) continue;
-#pragma unroll
-        for (int i = 0; i < TB; ++i) {
-          const int ii = bt * TB + i;
-          if (ii >= N) continue;
-          Cx* o = coarse + ((int64_t)c * nrhs + r) * N + ii;
-          if (accumulate) { Cx v = *o; v.x += acc[j][i].x; v.y += acc[j][i].y; *o = v; }
-          else *o = acc[j][i];
-        }
-      }
-    }
-  }
-}
+    for (int q = 0; q < RQ; ++q) acc[m][q][0] = acc[m][q][1] = 0.0;
 
-template <class T, int TR, int TB, int KS>
-static gmg_status launch_project(gmg_agg* h, const void* basis, int nrhs, const void* fine,
-                                 void* coarse, const int8_t* mask, int accumulate, cudaStream_t s,
-                                 const int32_t* sel = nullptr, int nsel = 0) {
-  typedef typename ctype<T>::t Cx;
-  const int N = h->N, R = nrhs;
-  const int ntiles = ((N + TB - 1) / TB) * ((R + TR - 1) / TR);
-  GMG_CHECK(ntiles <= 256, GMG_ERR_UNSUPPORTED, "project: nbasis x nrhs too large");
-  const int threads = std::max(32, (ntiles + 31) / 32 * 32);
-  const size_t smem = sizeof(Cx) * (size_t)KS * h->dof * (N + R);
-  GMG_CHECK(smem <= 227 * 1024, GMG_ERR_UNSUPPORTED, "project: shared-memory tile too large");
-  auto kern = project_kernel<T, TR, TB, KS>;
-  GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int Vc = (int)h->cdims.vol();
-  const int grid = std::min(Vc, num_sms() * 16);
-  KernelTimer kt("project", s);
-  kern<<<grid, threads, smem, s>>>(reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
-                                   reinterpret_cast<const Cx*>(fine), reinterpret_cast<Cx*>(coarse),
-                                   Vc, N, h->dof, h->bv, nrhs, mask, accumulate, sel, nsel);
-  GMG_CUDA(cudaGetLastError());
-  return GMG_OK;
-}
-
-// ---------------------------------------------------------------------------
-// FP64 projection of spin-colour fields (dof 12, nrhs >= 4), pipelined: the
-// same sums as project_kernel, with
-//   - the next KS-site chunk of basis and fine field copied into the second
-//     shared-memory buffer (cp.async, 16 B per complex number, written
-//     straight into the transposed [k][N] / [k][R] tiles) while the current
-//     one is multiplied, so the global loads no longer stall the FMA loop;
-//   - basis rows and RHS interleaved over the threads (thread (bt, rt) owns
-//     rows bt + NBT i and RHS rt + NRT j), so the 16-byte shared loads of
-//     neighbouring threads fall on consecutive banks;
-//   - the chunk's index arithmetic on compile-time strides.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
-               "l"(gmem)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N_>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_) : "memory"); }
-
-template <int DOF, int KS, int TR, int TB, int NT>
-__global__ void __launch_bounds__(NT, 384 / NT) project_f64_pipe_kernel(
-    const double2* __restrict__ basis, const int32_t* __restrict__ blk_sites, const double2* __restrict__ fine,
-    double2* __restrict__ coarse, int Vc, int N, int bv, int nrhs, const int32_t* __restrict__ sel, int nsel) {
-  constexpr int KC = KS * DOF;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int R = nrhs;
-  const int NBT = (N + TB - 1) / TB, NRT = (R + TR - 1) / TR;
-  // tile widths padded to whole register tiles; the pad columns are zeroed
-  // once and never copied to, so the multiply loop needs no bounds tests
-  const int Np = NBT * TB, Rq = NRT * TR;
-  double2* buf0 = reinterpret_cast<double2*>(smem_raw);  // per buffer: VT [KC][Np], FT [KC][Rq]
-  const int bufsz = KC * (Np + Rq);
-  const int ntiles = NBT * NRT;
-  const int t = threadIdx.x, bt = t % NBT, rt = t / NBT;
-  const int64_t K = (int64_t)bv * DOF;
-  const int nsites = sel ? nsel : bv;
-  const int nch = (nsites + KS - 1) / KS;
-  for (int e = t; e < 2 * bufsz; e += NT) buf0[e] = make_double2(0.0, 0.0);
-  for (int c = blockIdx.x; c < Vc; c += gridDim.x) {
-    const double2* Vb = basis + (int64_t)c * N * K;
-    // copies of chunk ch into buffer b (sites beyond nsites are skipped; the
-    // multiply loop stops at the chunk's own length)
-    auto issue = [&](int ch, int b) {
-      double2* VT = buf0 + b * bufsz;
-      double2* FT = VT + KC * Np;
-      const int sb0 = ch * KS;
-      const int ns = min(KS, nsites - sb0);
-      for (int e = t; e < N * KC; e += NT) {
-        const int i = e / KC, kk = e % KC;
-        const int sl = kk / DOF, a = kk % DOF;
-        if (sl < ns) {
-          const int sb = sel ? sel[sb0 + sl] : sb0 + sl;
-          cp_async16(VT + kk * Np + i, Vb + (int64_t)i * K + (int64_t)sb * DOF + a);
-        }
+  if (u < a.units && ks < nsites) {
+    // rows and right-hand sides past the end repeat the last one; their results are not stored
+    const Cx* Vb = a.basis + c * N * K;
+    const int32_t* blk = a.blk_sites + c * a.bv;
+    uint32_t row[MT];
+    int foff[RQ];
+    const uint32_t Kb = (uint32_t)(K * sizeof(Cx));
+#pragma unroll
+    for (int m = 0; m < MT; ++m) row[m] = min((mc * MT + m) * 8 + (lane >> 2), N - 1);
+#pragma unroll
+    for (int q = 0; q < RQ; ++q) foff[q] = min((rc * RQ + q) * 4 + (lane >> 3), a.nrhs - 1) * dof;
+    const uint32_t s1 = f64mma::second_sign(part, true);
+    Cx av[2][MT], fv[2][RQ];
+    int s = ks, k4 = 0, left = (nsites - ks + a.KS - 1) / a.KS * ((dof + 3) / 4);
+    // the site requested next and the one after it
+    int sb = a.sel ? a.sel[s] : s, sf = blk[sb];
+    int sb1 = 0, sf1 = 0;
+    const Cx *Vp, *Fp;
+    auto at_site = [&]() {
+      Vp = Vb + (int64_t)sb * dof;
+      Fp = a.fine + (int64_t)sf * a.nrhs * dof;
+      s += a.KS;
+      if (s < nsites) {
+        sb1 = a.sel ? a.sel[s] : s;
+        sf1 = blk[sb1];
       }
-      for (int sl = 0; sl < ns; ++sl) {
-        const int64_t sf = blk_sites[(int64_t)c * bv + (sel ? sel[sb0 + sl] : sb0 + sl)];
-        const double2* src = fine + sf * nrhs * DOF;
-        for (int e = t; e < R * DOF; e += NT) {
-          const int r = e / DOF, a = e % DOF;
-          cp_async16(FT + (sl * DOF + a) * Rq + r, src + e);
-        }
-      }
-      cp_async_commit();
     };
-    double2 acc[TR][TB];
+    auto request = [&](Cx (&A)[MT], Cx (&F)[RQ]) {
+      const int k = k4 + kk;
+      const bool in_k = k < dof;
 #pragma unroll
-    for (int j = 0; j < TR; ++j)
+      for (int m = 0; m < MT; ++m) A[m] = in_k ? __ldg(reinterpret_cast<const Cx*>(reinterpret_cast<const char*>(Vp + k) + (uint64_t)row[m] * Kb)) : Cx{0, 0};
 #pragma unroll
-      for (int i = 0; i < TB; ++i) acc[j][i] = make_double2(0.0, 0.0);
-    __syncthreads();  // zeroing done / the previous block's last chunk is no longer read
-    issue(0, 0);
-    for (int ch = 0; ch < nch; ++ch) {
-      if (ch + 1 < nch) {
-        issue(ch + 1, (ch + 1) & 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
+      for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(Fp + foff[q] + k) : Cx{0, 0};
+      k4 += 4;
+      if (k4 >= dof) {
+        k4 = 0;
+        sb = sb1;
+        sf = sf1;
+        at_site();
       }
-      __syncthreads();
-      const double2* va = buf0 + (ch & 1) * bufsz + bt;
-      const double2* xa = buf0 + (ch & 1) * bufsz + KC * Np + rt;
-      const int kc = min(KS, nsites - ch * KS) * DOF;
-      if (t < ntiles) {
-#pragma unroll 1
-        for (int kk = 0; kk < kc; ++kk) {
-          double2 a[TB], x[TR];
+    };
+    auto multiply = [&](const Cx (&A)[MT], const Cx (&F)[RQ]) {
+      double b0[RQ], b1[RQ];
 #pragma unroll
-          for (int i = 0; i < TB; ++i) a[i] = va[kk * Np + NBT * i];
+      for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, 0u, s1, b0[q], b1[q]);
 #pragma unroll
-          for (int j = 0; j < TR; ++j) x[j] = xa[kk * Rq + NRT * j];
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-          for (int j = 0; j < TR; ++j)
+        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].x, b0[q]);
 #pragma unroll
-            for (int i = 0; i < TB; ++i) acc[j][i] = cfma_conj(acc[j][i], a[i], x[j]);
-        }
-      }
-      __syncthreads();  // buffer (ch & 1) is refilled by the issue of chunk ch + 2
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].y, b1[q]);
+    };
+    at_site();
+    request(av[0], fv[0]);
+    for (;;) {
+      if (left > 1) request(av[1], fv[1]);
+      multiply(av[0], fv[0]);
+      if (--left == 0) break;
+      if (left > 1) request(av[0], fv[0]);
+      multiply(av[1], fv[1]);
+      if (--left == 0) break;
     }
-    if (t < ntiles) {
+  }
+
+  auto store = [&](int m, int q, double re, double im) {
+    const int i = (mc * MT + m) * 8 + (lane >> 2), r = (rc * RQ + q) * 4 + kk;
+    if (i >= N || r >= a.nrhs) return;
+    Cx v;
+    v.x = re;
+    v.y = im;
+    a.out[c * a.cstr + r * a.rstr + i * a.istr] = v;
+  };
+  if (a.KS == 1) {
+    if (u < a.units) {
 #pragma unroll
-      for (int j = 0; j < TR; ++j) {
-        const int r = rt + NRT * j;
-        if (r >= R) continue;
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int i = 0; i < TB; ++i) {
-          const int ii = bt + NBT * i;
-          if (ii < N) coarse[((int64_t)c * nrhs + r) * N + ii] = acc[j][i];
-        }
+        for (int q = 0; q < RQ; ++q) store(m, q, acc[m][q][0], acc[m][q][1]);
+    }
+    return;
+  }
+  double2* red = reinterpret_cast<double2*>(smem_raw) + (int64_t)g * a.KS * MT * RQ * 32;
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int q = 0; q < RQ; ++q)
+      red[(ks * MT * RQ + m * RQ + q) * 32 + lane] = make_double2(acc[m][q][0], acc[m][q][1]);
+  __syncthreads();
+  if (u < a.units) {
+    for (int t = ks; t < MT * RQ; t += a.KS) {
+      double re = 0.0, im = 0.0;
+      for (int j = 0; j < a.KS; ++j) {
+        const double2 v = red[(j * MT * RQ + t) * 32 + lane];
+        re += v.x;
+        im += v.y;
       }
+      store(t / RQ, t % RQ, re, im);
     }
   }
 }
 
-template <int KS, int TR, int TB, int NT>
-static gmg_status launch_pipe(gmg_agg* h, int nrhs, const void* fine, void* coarse, const int32_t* sel, int nsel,
-                              cudaStream_t s) {
-  const int N = h->N, R = nrhs;
-  const int Np = (N + TB - 1) / TB * TB, Rq = (R + TR - 1) / TR * TR;
-  const size_t smem = sizeof(double2) * 2 * (size_t)KS * 12 * (Np + Rq);
-  auto kern = project_f64_pipe_kernel<12, KS, TR, TB, NT>;
-  GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int Vc = (int)h->cdims.vol();
-  const int grid = std::min(Vc, num_sms() * 16);
+template <class T, int MT, int RQ>
+static gmg_status launch_project(const ProjArgs<typename ctype<T>::t>& a, int Vc, cudaStream_t s) {
+  auto kern = project_mma_kernel<T, MT, RQ>;
+  const size_t smem = a.KS == 1 ? 0 : sizeof(double2) * 32 * MT * RQ * (size_t)a.G * a.KS;
+  if (smem > 48 * 1024)
+    GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   KernelTimer kt("project", s);
-  kern<<<grid, NT, smem, s>>>(h->basis_blk.as<double2>(), h->blk_sites.as<int32_t>(),
-                              reinterpret_cast<const double2*>(fine), reinterpret_cast<double2*>(coarse), Vc, N, h->bv,
-                              nrhs, sel, nsel);
+  kern<<<dim3(Vc, (a.units + a.G - 1) / a.G), 32 * a.G * a.KS, smem, s>>>(a);
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
 
-// the pipelined FP64 projection when it applies (dof 12, 4 <= nrhs, tiles and
-// two buffers within limits); *launched = false otherwise.  5 x 5 register
-// tiles on 64 threads when they fill more than one warp with nbasis and nrhs
-// up to 40 (the coarsening's 40 x 40: 64 threads, no idle lanes), else 4 x 4
-// on 128 threads.
-static gmg_status launch_project_f64_pipe(gmg_agg* h, int nrhs, const void* fine, void* coarse, const int32_t* sel,
-                                          int nsel, cudaStream_t s, bool* launched) {
-  *launched = false;
-  const int N = h->N, R = nrhs;
-  if (h->dof != 12 || R < 4 || (reinterpret_cast<uintptr_t>(fine) & 15)) return GMG_OK;
-  const int t5 = ((N + 4) / 5) * ((R + 4) / 5);
-  if (N <= 40 && R <= 40 && t5 > 32) {
-    GMG_TRY((launch_pipe<1, 5, 5, 64>(h, nrhs, fine, coarse, sel, nsel, s)));
-  } else {
-    const int t4 = ((N + 3) / 4) * ((R + 3) / 4);
-    if (t4 > 128 || sizeof(double2) * 2 * 2 * 12 * (size_t)(N + R + 6) > 200 * 1024) return GMG_OK;
-    GMG_TRY((launch_pipe<2, 4, 4, 128>(h, nrhs, fine, coarse, sel, nsel, s)));
+// Launch shape of the projection: w quads of right-hand sides per unit, G units
+// and KS shares of the sites per CTA.  The grid's time in units of MMA work is
+// estimated for every w, with the units of a block in one CTA (their operands
+// meet in L1) or in CTAs of their own: CTAs in full waves of C per SM, the last
+// wave with what is left; the basis read of a unit counts as half a quad, 0.4
+// when shared.  Big tiles run in CTAs of 4 warps, so that two or three CTAs
+// overlap each other's ends (32^4, nbasis 32, 32 RHS, FP64: 3.71 ms, 5.12 with
+// 8), small tiles and part-filled chips in CTAs of 8 (16^4, nbasis 24, 12 RHS:
+// 95 us, 118 with 4).  16^4, nbasis 32, 32 RHS: 290 us with w = 2 and own CTAs,
+// 376 with w = 4 and shared ones; 8^4 with 16 blocks, nbasis 24, 24 RHS: 37 us
+// with w = 1, 98 with w = 3.
+struct ProjShape {
+  int w, chunks, G, KS;
+};
+static ProjShape project_shape(int Vc, int MT, int mchunks, int rq) {
+  ProjShape best{1, rq, 1, kProjWarps};
+  double t_best = 1e30;
+  for (int w = 1; w <= std::min(5, rq); ++w) {
+    const int chunks = (rq + w - 1) / w, units = mchunks * chunks;
+    const int regs = (40 + 4 * MT * w + 8 * MT + 8 * w + 7) / 8 * 8;
+    for (int shared = 0; shared < 2; ++shared) {
+      int warps = MT * w > 10 ? 4 : kProjWarps;
+      int G = shared ? std::min(units, warps) : 1;
+      int64_t ctas = (int64_t)Vc * ((units + G - 1) / G);
+      if (ctas < 2 * 148) {
+        warps = kProjWarps;
+        G = shared ? std::min(units, warps) : 1;
+        ctas = (int64_t)Vc * ((units + G - 1) / G);
+      }
+      const int C = std::max(1, 65536 / 32 / regs / warps);
+      const double work = G * MT * (w + (G > 1 ? 0.4 : 0.5)) * (C > 1 ? 1.0 : 1.25);
+      const int64_t rest = ctas % (148 * C);
+      const double t = work * (ctas / (148 * C) * C + (rest + 147) / 148);
+      if (t <= t_best) {
+        t_best = t;
+        best = ProjShape{w, chunks, G, warps / G};
+      }
+    }
   }
-  *launched = true;
-  return GMG_OK;
+  return best;
 }
 
-gmg_status agg_project(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* fine,
-                       void* coarse, const int32_t* mask_unused, cudaStream_t s) {
-  (void)mask_unused;
+template <class T>
+static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const void* fine, void* out, int64_t cstr,
+                              int64_t rstr, int64_t istr, const int32_t* sel, int nsel, cudaStream_t s) {
+  typedef typename ctype<T>::t Cx;
+  GMG_CHECK(sizeof(Cx) * 4 * h->dof * (size_t)(h->N + nrhs) <= 227 * 1024, GMG_ERR_UNSUPPORTED,
+            "project: site dof x (nbasis + nrhs) too large");
+  GMG_CHECK((int64_t)h->bv * h->dof < ((int64_t)1 << 28), GMG_ERR_UNSUPPORTED, "project: more than 2^28 components per block");
+  const int mt = (h->N + 7) / 8, mchunks = (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
+  const int Vc = (int)h->cdims.vol();
+  const ProjShape sh = project_shape(Vc, MT, mchunks, (nrhs + 3) / 4);
+  const ProjArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
+                       reinterpret_cast<const Cx*>(fine), reinterpret_cast<Cx*>(out), cstr, rstr, istr, h->N, h->dof,
+                       h->bv, nrhs, sel, nsel, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
+  auto by_rq = [&](auto mtc) -> gmg_status {
+    constexpr int M = decltype(mtc)::value;
+    switch (sh.w) {
+      case 1: return launch_project<T, M, 1>(a, Vc, s);
+      case 2: return launch_project<T, M, 2>(a, Vc, s);
+      case 3: return launch_project<T, M, 3>(a, Vc, s);
+      case 4: return launch_project<T, M, 4>(a, Vc, s);
+      default: return launch_project<T, M, 5>(a, Vc, s);
+    }
+  };
+  switch (MT) {
+    case 1: return by_rq(std::integral_constant<int, 1>());
+    case 2: return by_rq(std::integral_constant<int, 2>());
+    case 3: return by_rq(std::integral_constant<int, 3>());
+    case 4: return by_rq(std::integral_constant<int, 4>());
+    default: return by_rq(std::integral_constant<int, 5>());
+  }
+}
+
+gmg_status agg_project(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* fine, void* coarse,
+                       cudaStream_t s) {
   if (compute == GMG_BF16 && vec_prec == GMG_F32) return agg_project_tc(h, nrhs, (const float*)fine, (float*)coarse, s);
   GMG_CHECK(compute == vec_prec, GMG_ERR_UNSUPPORTED, "project: compute and vector precision differ");
-  if (compute == GMG_F64) {
-    bool done = false;
-    GMG_TRY(launch_project_f64_pipe(h, nrhs, fine, coarse, nullptr, 0, s, &done));
-    if (done) return GMG_OK;
-    if (nrhs >= 4) return launch_project<double, 4, 4, 4>(h, h->basis_blk.p, nrhs, fine, coarse, nullptr, 0, s);
-    return launch_project<double, 1, 2, 4>(h, h->basis_blk.p, nrhs, fine, coarse, nullptr, 0, s);
-  }
+  const int64_t N = h->N;
+  if (compute == GMG_F64)
+    return project_mma<double>(h, h->basis_blk.p, nrhs, fine, coarse, nrhs * N, N, 1, nullptr, 0, s);
   if (compute == GMG_F32) {
     GMG_TRY(agg_prepare_f32(h, s));
-    if (nrhs >= 4) return launch_project<float, 4, 4, 4>(h, h->basis_blk_f.p, nrhs, fine, coarse, nullptr, 0, s);
-    return launch_project<float, 1, 2, 4>(h, h->basis_blk_f.p, nrhs, fine, coarse, nullptr, 0, s);
+    return project_mma<float>(h, h->basis_blk_f.p, nrhs, fine, coarse, nrhs * N, N, 1, nullptr, 0, s);
   }
   return fail(GMG_ERR_UNSUPPORTED, "project: unsupported precision");
 }
 
 // FP64 projection over a subset of every block's sites (sel: nsel in-block
-// indices on the device, the same for all blocks), used for the face terms of
-// the coarse-operator construction
-gmg_status agg_project_sel_f64(gmg_agg* h, int nrhs, const double* fine, double* coarse, const int32_t* sel,
-                               int nsel, cudaStream_t s) {
-  bool done = false;
-  GMG_TRY(launch_project_f64_pipe(h, nrhs, fine, coarse, sel, nsel, s, &done));
-  if (done) return GMG_OK;
-  if (nrhs >= 4)
-    return launch_project<double, 4, 4, 4>(h, h->basis_blk.p, nrhs, fine, coarse, nullptr, 0, s, sel, nsel);
-  return launch_project<double, 1, 2, 4>(h, h->basis_blk.p, nrhs, fine, coarse, nullptr, 0, s, sel, nsel);
-}
-
-// masked FP64 single-RHS projection used by the coarse-operator construction
-gmg_status agg_project_masked_f64(gmg_agg* h, int nrhs, const double* fine, double* coarse,
-                                  const int8_t* mask, cudaStream_t s) {
-  if (!mask) {
-    bool done = false;
-    GMG_TRY(launch_project_f64_pipe(h, nrhs, fine, coarse, nullptr, 0, s, &done));
-    if (done) return GMG_OK;
-  }
-  if (nrhs >= 4) return launch_project<double, 4, 4, 4>(h, h->basis_blk.p, nrhs, fine, coarse, mask, 0, s);
-  return launch_project<double, 1, 2, 4>(h, h->basis_blk.p, nrhs, fine, coarse, mask, 0, s);
+// indices on the device, the same for all blocks; null: all of them), written
+// as columns i0 .. i0 + nrhs of the link matrices A[c][i][column]
+gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, double* A, int i0, const int32_t* sel, int nsel,
+                             cudaStream_t s) {
+  const int64_t N = h->N;
+  return project_mma<double>(h, h->basis_blk.p, nrhs, fine, reinterpret_cast<double2*>(A) + i0, N * N, 1, N, sel, nsel,
+                             s);
 }
 
 // ---------------------------------------------------------------------------
 // promote: F[site(c,k)][r][k%dof] = sum_i V[c][i][k] C[c][r][i]
+// on the FP64 tensor cores: rows k (8 KT per warp and turn), contraction i.  A
+// block's coarse vectors are expanded once per CTA into MMA operand order in
+// shared memory; the basis is read straight from global memory, each element
+// once per chunk of 4 RQ right-hand sides, one step ahead.
+// What bounds it: the MMA rate, as the projection.  32^4, nbasis 32, 32 RHS,
+// 4^4 blocks, FP64: 9.64 -> 3.52 ms (29 TFLOP/s of 37); 16^4, nbasis 24, 12 RHS:
+// 946 -> 96 us.
 // ---------------------------------------------------------------------------
-template <class T, int TK, int TR, int KS>
-__global__ void __launch_bounds__(256) promote_kernel(
-    const typename ctype<T>::t* __restrict__ basis, const int32_t* __restrict__ blk_sites,
-    const typename ctype<T>::t* __restrict__ coarse, typename ctype<T>::t* __restrict__ fine, int Vc,
-    int N, int dof, int bv, int nrhs) {
+template <class Cx> struct PromArgs {
+  const Cx* basis;
+  const int32_t* blk_sites;
+  const Cx* coarse;
+  Cx* fine;
+  int N, dof, bv, nrhs, rq;  // rq: quads of the shared-memory table
+};
+
+template <class T, int KT, int RQ>
+__global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int KC = KS * dof;
-  const int R = nrhs;
-  Cx* CT = reinterpret_cast<Cx*>(smem_raw);  // [N][R]
-  Cx* VS = CT + N * R;                        // [N][KC]
-  const int NKT = KC / TK, NRT = (R + TR - 1) / TR;
-  const int ntiles = NKT * NRT;
-  const int t = threadIdx.x;
-  const int64_t K = (int64_t)bv * dof;
-  for (int c = blockIdx.x; c < Vc; c += gridDim.x) {
-    __syncthreads();
-    for (int e = t; e < N * R; e += blockDim.x) {
-      const int r = e / N, i = e % N;
-      CT[i * R + r] = coarse[((int64_t)c * nrhs + r) * N + i];
+  double2* Bs = reinterpret_cast<double2*>(smem_raw);  // [steps][rq][32]: (first, second) operand of every lane
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kk = lane & 3;
+  const int N = a.N, dof = a.dof, steps = (N + 3) / 4;
+  const int64_t c = blockIdx.x;
+  const int K = a.bv * dof;
+  for (int e = threadIdx.x; e < steps * a.rq * 32; e += blockDim.x) {
+    const int l = e & 31, q = (e >> 5) % a.rq, st = (e >> 5) / a.rq;
+    const int i = 4 * st + (l & 3), r = q * 4 + (l >> 3), part = (l >> 2) & 1;
+    Cx v{0, 0};
+    if (i < N && r < a.nrhs) v = a.coarse[(c * a.nrhs + r) * N + i];
+    double2 b;
+    f64mma::expand(v, part, 0u, f64mma::second_sign(part, false), b.x, b.y);
+    Bs[e] = b;
+  }
+  __syncthreads();
+  const Cx* Vb = a.basis + c * N * (int64_t)K;
+  const int32_t* blk = a.blk_sites + c * a.bv;
+  const int ngroups = (K + 8 * KT - 1) / (8 * KT), nwarps = (blockDim.x >> 5) * gridDim.y;
+  const int chunks = a.rq / RQ;
+  for (int item = blockIdx.y * (blockDim.x >> 5) + warp; item < ngroups * chunks; item += nwarps) {
+    const int grp = item / chunks, q0 = (item - grp * chunks) * RQ;
+    double acc[KT][RQ][2];
+#pragma unroll
+    for (int t = 0; t < KT; ++t)
+#pragma unroll
+      for (int q = 0; q < RQ; ++q) acc[t][q][0] = acc[t][q][1] = 0.0;
+    const int k0 = grp * 8 * KT + (lane >> 2);
+    int sf[KT], at[KT];  // site and component of this lane's rows
+    const Cx* Vp[KT];
+#pragma unroll
+    for (int t = 0; t < KT; ++t) {
+      const int k = min(k0 + 8 * t, K - 1);
+      const int sb = k / dof;
+      sf[t] = blk[sb];
+      at[t] = k - sb * dof;
+      Vp[t] = Vb + k;
     }
-    const Cx* Vb = basis + (int64_t)c * N * K;
-    for (int sb0 = 0; sb0 < bv; sb0 += KS) {
-      const int ns = min(KS, bv - sb0);
-      const int kc = ns * dof;
-      __syncthreads();
-      for (int e = t; e < N * kc; e += blockDim.x) {
-        const int i = e / kc, kk = e % kc;
-        VS[i * KC + kk] = Vb[(int64_t)i * K + (int64_t)sb0 * dof + kk];
+    Cx av[2][KT];
+    auto request = [&](Cx (&A)[KT], int st) {
+      const int i = 4 * st + kk;
+#pragma unroll
+      for (int t = 0; t < KT; ++t) A[t] = i < N ? __ldg(Vp[t] + (int64_t)i * K) : Cx{0, 0};
+    };
+    auto multiply = [&](const Cx (&A)[KT], int st) {
+      const double2* B = Bs + (st * a.rq + q0) * 32 + lane;
+#pragma unroll
+      for (int q = 0; q < RQ; ++q) {
+        const double2 b = B[q * 32];
+#pragma unroll
+        for (int t = 0; t < KT; ++t) f64mma::mma(acc[t][q], (double)A[t].x, b.x);
+#pragma unroll
+        for (int t = 0; t < KT; ++t) f64mma::mma(acc[t][q], (double)A[t].y, b.y);
       }
-      __syncthreads();
-      for (int tile = t; tile < ntiles; tile += blockDim.x) {
-        const int kt = tile % NKT, rt = tile / NKT;
-        if (kt * TK >= kc) continue;
-        Cx acc[TR][TK];
+    };
+    request(av[0], 0);
+    for (int st = 0; st < steps; st += 2) {
+      if (st + 1 < steps) request(av[1], st + 1);
+      multiply(av[0], st);
+      if (st + 1 == steps) break;
+      if (st + 2 < steps) request(av[0], st + 2);
+      multiply(av[1], st + 1);
+    }
 #pragma unroll
-        for (int j = 0; j < TR; ++j)
+    for (int t = 0; t < KT; ++t) {
+      if (k0 + 8 * t >= K) continue;
 #pragma unroll
-          for (int q = 0; q < TK; ++q) acc[j][q] = Cx{0, 0};
-        for (int i = 0; i < N; ++i) {
-          Cx v[TK], x[TR];
-#pragma unroll
-          for (int q = 0; q < TK; ++q) v[q] = VS[i * KC + kt * TK + q];
-#pragma unroll
-          for (int j = 0; j < TR; ++j) {
-            const int r = rt * TR + j;
-            x[j] = r < R ? CT[i * R + r] : Cx{0, 0};
-          }
-#pragma unroll
-          for (int j = 0; j < TR; ++j)
-#pragma unroll
-            for (int q = 0; q < TK; ++q) acc[j][q] = cfma(acc[j][q], x[j], v[q]);
-        }
-        const int k0 = kt * TK;
-        const int sl = k0 / dof, a0 = k0 % dof;  // TK divides dof: one site per tile
-        const int sf = blk_sites[(int64_t)c * bv + sb0 + sl];
-#pragma unroll
-        for (int j = 0; j < TR; ++j) {
-          const int r = rt * TR + j;
-          if (r >= R) continue;
-          Cx* o = fine + ((int64_t)sf * nrhs + r) * dof + a0;
-#pragma unroll
-          for (int q = 0; q < TK; ++q) o[q] = acc[j][q];
-        }
+      for (int q = 0; q < RQ; ++q) {
+        const int r = (q0 + q) * 4 + kk;
+        if (r >= a.nrhs) continue;
+        Cx v;
+        v.x = acc[t][q][0];
+        v.y = acc[t][q][1];
+        a.fine[((int64_t)sf[t] * a.nrhs + r) * dof + at[t]] = v;
       }
     }
   }
 }
 
-template <class T, int TK, int TR, int KS>
-static gmg_status launch_promote(gmg_agg* h, const void* basis, int nrhs, const void* coarse,
-                                 void* fine, cudaStream_t s) {
-  typedef typename ctype<T>::t Cx;
-  const int N = h->N, R = nrhs, dof = h->dof;
-  GMG_CHECK(dof % TK == 0, GMG_ERR_UNSUPPORTED, "promote: dof not a multiple of the k tile");
-  const int ntiles = (KS * dof / TK) * ((R + TR - 1) / TR);
-  const int threads = std::min(256, std::max(32, (ntiles + 31) / 32 * 32));
-  const size_t smem = sizeof(Cx) * ((size_t)N * R + (size_t)N * KS * dof);
-  GMG_CHECK(smem <= 227 * 1024, GMG_ERR_UNSUPPORTED, "promote: shared-memory tile too large");
-  auto kern = promote_kernel<T, TK, TR, KS>;
-  GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int Vc = (int)h->cdims.vol();
-  const int grid = std::min(Vc, num_sms() * 16);
+template <class T, int KT, int RQ>
+static gmg_status launch_promote(PromArgs<typename ctype<T>::t> a, int Vc, cudaStream_t s) {
+  auto kern = promote_mma_kernel<T, KT, RQ>;
+  const size_t smem = sizeof(double2) * 32 * (size_t)((a.N + 3) / 4) * a.rq;
+  if (smem > 48 * 1024)
+    GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // 8 warps per CTA; few blocks are split over several CTAs, up to 6 per SM with
+  // 3 turns a warp or more (256 blocks, nbasis 32, 32 RHS: 252 us at 4, 276 at 1;
+  // 16 blocks, nbasis 24, 24 RHS: 18 us at 8, 97 at 1)
+  const int items = (a.bv * a.dof + 8 * KT - 1) / (8 * KT) * (a.rq / RQ);
+  const int split = std::max(1, std::min((items + 23) / 24, (148 * 6 + Vc - 1) / Vc));
   KernelTimer kt("promote", s);
-  kern<<<grid, threads, smem, s>>>(reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
-                                   reinterpret_cast<const Cx*>(coarse), reinterpret_cast<Cx*>(fine),
-                                   Vc, N, dof, h->bv, nrhs);
+  kern<<<dim3(Vc, split), 256, smem, s>>>(a);
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
+}
+
+template <class T>
+static gmg_status promote_mma(gmg_agg* h, const void* basis, int nrhs, const void* coarse, void* fine,
+                              cudaStream_t s) {
+  typedef typename ctype<T>::t Cx;
+  GMG_CHECK(sizeof(Cx) * ((size_t)h->N * nrhs + (size_t)h->N * 4 * h->dof) <= 227 * 1024, GMG_ERR_UNSUPPORTED,
+            "promote: nbasis x (nrhs + site dof) too large");
+  GMG_CHECK((int64_t)h->bv * h->dof < ((int64_t)1 << 28), GMG_ERR_UNSUPPORTED, "promote: more than 2^28 components per block");
+  // quads per warp: the fewest padded ones (each chunk reads the basis once
+  // more, counted as half a quad)
+  const int rq = (nrhs + 3) / 4;
+  int w = 1, chunks = rq;
+  for (int v = 2; v <= 8; ++v) {
+    const int u = (rq + v - 1) / v;
+    if (u * (2 * v + 1) <= chunks * (2 * w + 1)) {
+      w = v;
+      chunks = u;
+    }
+  }
+  PromArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(), reinterpret_cast<const Cx*>(coarse),
+                 reinterpret_cast<Cx*>(fine), h->N, h->dof, h->bv, nrhs, w * chunks};
+  const int Vc = (int)h->cdims.vol();
+  switch (w) {
+    case 1: return launch_promote<T, 4, 1>(a, Vc, s);
+    case 2: return launch_promote<T, 4, 2>(a, Vc, s);
+    case 3: return launch_promote<T, 4, 3>(a, Vc, s);
+    case 4: return launch_promote<T, 4, 4>(a, Vc, s);
+    case 5: return launch_promote<T, 3, 5>(a, Vc, s);
+    case 6: return launch_promote<T, 2, 6>(a, Vc, s);
+    case 7: return launch_promote<T, 2, 7>(a, Vc, s);
+    default: return launch_promote<T, 2, 8>(a, Vc, s);
+  }
 }
 
 gmg_status agg_promote(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* coarse,
                        void* fine, cudaStream_t s) {
   if (compute == GMG_BF16 && vec_prec == GMG_F32) return agg_promote_tc(h, nrhs, (const float*)coarse, (float*)fine, s);
   GMG_CHECK(compute == vec_prec, GMG_ERR_UNSUPPORTED, "promote: compute and vector precision differ");
-  const bool tk4 = h->dof % 4 == 0;
-  if (compute == GMG_F64) {
-    if (nrhs >= 4 && tk4) return launch_promote<double, 4, 4, 4>(h, h->basis_blk.p, nrhs, coarse, fine, s);
-    if (tk4) return launch_promote<double, 4, 1, 4>(h, h->basis_blk.p, nrhs, coarse, fine, s);
-    return launch_promote<double, 1, 1, 4>(h, h->basis_blk.p, nrhs, coarse, fine, s);
-  }
+  if (compute == GMG_F64) return promote_mma<double>(h, h->basis_blk.p, nrhs, coarse, fine, s);
   if (compute == GMG_F32) {
     GMG_TRY(agg_prepare_f32(h, s));
-    if (nrhs >= 4 && tk4) return launch_promote<float, 4, 4, 4>(h, h->basis_blk_f.p, nrhs, coarse, fine, s);
-    if (tk4) return launch_promote<float, 4, 1, 4>(h, h->basis_blk_f.p, nrhs, coarse, fine, s);
-    return launch_promote<float, 1, 1, 4>(h, h->basis_blk_f.p, nrhs, coarse, fine, s);
+    return promote_mma<float>(h, h->basis_blk_f.p, nrhs, coarse, fine, s);
   }
   return fail(GMG_ERR_UNSUPPORTED, "promote: unsupported precision");
 }

@@ -296,7 +296,7 @@ struct MmaShape {
 };
 static MmaShape mma_shape(int64_t nsites, int npts, int MT, int mchunks, int rq) {
   MmaShape sh{1, rq, 1, 1};
-  for (int w = 2; w <= 4; ++w) {
+  for (int w = 2; w <= 5; ++w) {
     const int u = (rq + w - 1) / w;
     if (u * (2 * w + 1) <= sh.chunks * (2 * sh.w + 1)) sh = MmaShape{w, u, 1, 1};
   }
@@ -328,7 +328,8 @@ static gmg_status coarse_mma(const LinkSel& L, const void* in, void* out, int V,
       case 1: return launch_mma<T, M, 1>(a, nsites, s);
       case 2: return launch_mma<T, M, 2>(a, nsites, s);
       case 3: return launch_mma<T, M, 3>(a, nsites, s);
-      default: return launch_mma<T, M, 4>(a, nsites, s);
+      case 4: return launch_mma<T, M, 4>(a, nsites, s);
+      default: return launch_mma<T, M, 5>(a, nsites, s);
     }
   };
   switch (MT) {

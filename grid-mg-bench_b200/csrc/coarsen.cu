@@ -20,11 +20,6 @@
 
 namespace gmg {
 
-gmg_status agg_project_masked_f64(gmg_agg* h, int nrhs, const double* fine, double* coarse,
-                                  const int8_t* mask, cudaStream_t s);
-gmg_status agg_project_sel_f64(gmg_agg* h, int nrhs, const double* fine, double* coarse, const int32_t* sel,
-                               int nsel, cudaStream_t s);
-
 // field[sf][r][a] = basis_blk[c][i0 + r][sb*dof + a]
 __global__ void basis_gather_kernel(const double2* __restrict__ basis_blk, const int32_t* __restrict__ blk_sites,
                                     double2* __restrict__ field, int64_t Vc, int N, int bv, int dof, int i0,
@@ -60,19 +55,6 @@ __global__ void mask_merge_kernel(const double2* __restrict__ a, const double2* 
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x)
     out[e] = mask[e / width] ? a[e] : b[e];
-}
-
-// A_p(c)[j][i0 + r] = proj[c][r][j]
-__global__ void link_scatter_kernel(const double2* __restrict__ proj, double2* __restrict__ A, int64_t Vc,
-                                    int N, int i0, int nb) {
-  const int64_t total = Vc * nb * N;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e % N);
-    const int r = (int)((e / N) % nb);
-    const int64_t c = e / ((int64_t)N * nb);
-    A[(c * N + j) * N + i0 + r] = proj[e];
-  }
 }
 
 static int gsz(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n + 255) / 256, 1), 148 * 64); }
@@ -135,12 +117,11 @@ static gmg_status coarsen_generic(gmg_coarse* out, gmg_agg* agg, const FineOpRef
   while (nb > 1 && (double)Vf * nb * dof * 16.0 > cap) nb = (nb + 1) / 2;
   if (agg->cw_max_batch > 0) nb = std::min(nb, agg->cw_max_batch);
   const size_t fbytes = sizeof(double2) * (size_t)Vf * nb * dof;
-  DevBuf phi, w1, w2, w3, proj, masks;
+  DevBuf phi, w1, w2, w3, masks;
   GMG_TRY(phi.alloc(fbytes));
   GMG_TRY(w1.alloc(fbytes));
   GMG_TRY(w2.alloc(fbytes));
   GMG_TRY(w3.alloc(fbytes));
-  GMG_TRY(proj.alloc(sizeof(double2) * (size_t)Vc * nb * N));
   std::vector<int8_t> hm;
   host_masks(fd, agg->b, hm);
   GMG_TRY(masks.alloc(hm.size()));
@@ -178,11 +159,8 @@ static gmg_status coarsen_generic(gmg_coarse* out, gmg_agg* agg, const FineOpRef
     GMG_CUDA(cudaGetLastError());
     for (int p = 4; p < 8; ++p) {
       GMG_TRY(op.mdir(p, cur, phi.as<double>(), w1.as<double>(), s));
-      GMG_TRY(agg_project_sel_f64(agg, cur, w1.as<double>(), proj.as<double>(), sel.as<int32_t>() + sel_off[p - 4],
-                                  nsel[p - 4], s));
-      link_scatter_kernel<<<gsz(Vc * cur * N), 256, 0, s>>>(proj.as<double2>(), A + (int64_t)p * Vc * N * N,
-                                                             Vc, N, i0, cur);
-      GMG_CUDA(cudaGetLastError());
+      GMG_TRY(agg_project_links(agg, cur, w1.as<double>(), reinterpret_cast<double*>(A + (int64_t)p * Vc * N * N), i0,
+                                sel.as<int32_t>() + sel_off[p - 4], nsel[p - 4], s));
     }
     // self term
     mask_select_kernel<<<gsz(Vf * wdt), 256, 0, s>>>(phi.as<double2>(), w1.as<double2>(), even, Vf, wdt, 1);
@@ -192,10 +170,8 @@ static gmg_status coarsen_generic(gmg_coarse* out, gmg_agg* agg, const FineOpRef
     mask_merge_kernel<<<gsz(Vf * wdt), 256, 0, s>>>(w2.as<double2>(), w3.as<double2>(), w1.as<double2>(), even,
                                                     Vf, wdt);
     GMG_CUDA(cudaGetLastError());
-    GMG_TRY(agg_project_masked_f64(agg, cur, w1.as<double>(), proj.as<double>(), nullptr, s));
-    link_scatter_kernel<<<gsz(Vc * cur * N), 256, 0, s>>>(proj.as<double2>(), A + (int64_t)8 * Vc * N * N, Vc,
-                                                           N, i0, cur);
-    GMG_CUDA(cudaGetLastError());
+    GMG_TRY(agg_project_links(agg, cur, w1.as<double>(), reinterpret_cast<double*>(A + (int64_t)8 * Vc * N * N), i0,
+                              nullptr, 0, s));
   }
   (void)width;
   GMG_TRY(coarse_construct_remaining(out, s));
@@ -216,7 +192,7 @@ static gmg_status coarsen_generic(gmg_coarse* out, gmg_agg* agg, const FineOpRef
 static gmg_status coarsen_workspace(gmg_agg* agg, cudaStream_t s) {
   if (agg->cw_nb > 0) return GMG_OK;
   const Dims& fd = agg->fdims;
-  const int64_t Vf = fd.vol(), Vc = agg->cdims.vol();
+  const int64_t Vf = fd.vol();
   const int N = agg->N, dof = agg->dof;
   size_t free_b = 0, total_b = 0;
   GMG_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -227,7 +203,6 @@ static gmg_status coarsen_workspace(gmg_agg* agg, cudaStream_t s) {
   const size_t fbytes = sizeof(double2) * (size_t)Vf * nb * dof;
   GMG_TRY(agg->cw_phi.alloc(fbytes));
   GMG_TRY(agg->cw_w.alloc(fbytes));
-  GMG_TRY(agg->cw_proj.alloc(sizeof(double2) * (size_t)Vc * nb * N));
   std::vector<int32_t> face, sel;
   std::vector<uint8_t> bpar(Vf), hskip(Vf);
   for (int d = 0; d < 4; ++d) {
@@ -314,7 +289,6 @@ static gmg_status coarsen_wilson_faces(gmg_coarse* out, gmg_agg* agg, gmg_wilson
   const int nb = agg->cw_nb;
   double* phi = agg->cw_phi.as<double>();
   double* wf = agg->cw_w.as<double>();
-  double* proj = agg->cw_proj.as<double>();
   const int32_t* face = agg->cw_face.as<int32_t>();
   const int32_t* sel = agg->cw_sel.as<int32_t>();
   double2* A = out->links_ref.as<double2>();
@@ -327,18 +301,13 @@ static gmg_status coarsen_wilson_faces(gmg_coarse* out, gmg_agg* agg, gmg_wilson
     int fo = 0, so = 0;
     for (int d = 0; d < 4; ++d) {
       GMG_TRY(wilson_apply_face(w, 4 + d, cur, phi, wf, face + fo, agg->cw_nface[d], s));
-      GMG_TRY(agg_project_sel_f64(agg, cur, wf, proj, sel + so, agg->cw_nsel[d], s));
-      link_scatter_kernel<<<gsz(Vc * cur * N), 256, 0, s>>>(reinterpret_cast<const double2*>(proj),
-                                                             A + (int64_t)(4 + d) * Vc * N * N, Vc, N, i0, cur);
-      GMG_CUDA(cudaGetLastError());
+      GMG_TRY(agg_project_links(agg, cur, wf, reinterpret_cast<double*>(A + (int64_t)(4 + d) * Vc * N * N), i0, sel + so,
+                                agg->cw_nsel[d], s));
       fo += agg->cw_nface[d];
       so += agg->cw_nsel[d];
     }
     GMG_TRY(wilson_apply_sel(w, GMG_OP_M, 0, 0, cur, phi, wf, nullptr, 0, agg->cw_hskip.as<uint8_t>(), s));
-    GMG_TRY(agg_project_masked_f64(agg, cur, wf, proj, nullptr, s));
-    link_scatter_kernel<<<gsz(Vc * cur * N), 256, 0, s>>>(reinterpret_cast<const double2*>(proj),
-                                                           A + (int64_t)8 * Vc * N * N, Vc, N, i0, cur);
-    GMG_CUDA(cudaGetLastError());
+    GMG_TRY(agg_project_links(agg, cur, wf, reinterpret_cast<double*>(A + (int64_t)8 * Vc * N * N), i0, nullptr, 0, s));
   }
   GMG_TRY(coarse_construct_remaining(out, s));
   GMG_TRY(coarse_links_to_site_major(out, s));

@@ -130,7 +130,7 @@ struct gmg_agg {
   // projection output, per direction the fine sites of the backward faces
   // (global, cw_face) and their in-block indices (cw_sel), and per site the
   // hops (bit p) whose neighbour lies in a block of the other parity (cw_hskip)
-  gmg::DevBuf cw_phi, cw_w, cw_proj, cw_face, cw_sel, cw_hskip;
+  gmg::DevBuf cw_phi, cw_w, cw_face, cw_sel, cw_hskip;
   int cw_nb = 0;
   int cw_max_batch = 0;  // cap on basis vectors per CoarsenOperator batch (0: from free memory)
   int cw_nface[4] = {0, 0, 0, 0}, cw_nsel[4] = {0, 0, 0, 0};
@@ -196,7 +196,9 @@ gmg_status agg_build_tables(gmg_agg* h, cudaStream_t s);
 gmg_status agg_basis_to_blocked(gmg_agg* h, const double* basis_dev, cudaStream_t s);
 gmg_status agg_basis_from_blocked(gmg_agg* h, double* basis_dev, cudaStream_t s);
 gmg_status agg_project(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* fine,
-                       void* coarse, const int32_t* mask_blk, cudaStream_t s);
+                       void* coarse, cudaStream_t s);
+gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, double* A, int i0, const int32_t* sel, int nsel,
+                             cudaStream_t s);
 gmg_status agg_promote(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* coarse,
                        void* fine, cudaStream_t s);
 // block orthonormalisation and its check (ortho.cu)

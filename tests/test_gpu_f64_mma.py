@@ -71,3 +71,30 @@ def test_stencil_active_list():
             assert orc.rel_dev_sq(ref[:, q], got[:, q]) < 1e-15
         else:
             assert np.all(got[:, q] == 7.0)
+
+
+@pytest.mark.parametrize("dt", [torch.complex128, torch.complex64])
+@pytest.mark.parametrize("fd,cd,dof,N,R", [
+    ((4, 4, 4, 4), (2, 2, 2, 2), 12, 2, 1),     # partial tiles of rows and right-hand sides
+    ((8, 8, 8, 4), (2, 2, 2, 1), 12, 8, 4),     # exactly one tile, few blocks
+    ((6, 4, 6, 4), (2, 2, 2, 2), 10, 18, 7),    # dof not a multiple of 4, block sizes 3 and 2
+    ((4, 4, 4, 2), (2, 2, 2, 2), 7, 5, 6),      # odd dof and nbasis; K = 56
+    ((3, 3, 2, 2), (3, 3, 2, 2), 12, 3, 5),     # one site per block: fewer sites than warps
+    ((8, 8, 8, 8), (4, 4, 4, 4), 12, 40, 21),   # five row tiles, six quads in chunks
+    ((4, 4, 4, 4), (2, 2, 2, 2), 40, 48, 33),   # two row chunks, nine quads
+    ((8, 8, 8, 8), (4, 8, 8, 8), 12, 24, 30),   # many small blocks
+])
+def test_project_and_promote(fd, cd, dof, N, R, dt):
+    Vf, Vc = int(np.prod(fd)), int(np.prod(cd))
+    r = inputs.rng(stream=710 + N + R)
+    B = inputs.gaussian_field((N, Vf, dof), r)
+    f = inputs.gaussian_field((Vf, R, dof), r)
+    c = inputs.gaussian_field((Vc, R, N), r)
+    ag = gmg.Aggregation(fd, cd, dof, N)
+    ag.set_basis(B)
+    got_c = torch.full((Vc, R, N), float("nan"), dtype=dt, device="cuda")  # every entry is written
+    got_f = torch.full((Vf, R, dof), float("nan"), dtype=dt, device="cuda")
+    ag.ProjectToSubspace(_dev(f, dt), got_c)
+    ag.PromoteFromSubspace(_dev(c, dt), got_f)
+    assert orc.rel_dev_sq(orc.block_project(fd, cd, B, f), _host(got_c)) < TOL[dt]
+    assert orc.rel_dev_sq(orc.block_promote(fd, cd, B, c), _host(got_f)) < TOL[dt]
