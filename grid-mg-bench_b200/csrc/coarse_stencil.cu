@@ -732,6 +732,15 @@ gmg_status coarse_apply_simt(gmg_coarse* h, int p0, int p1, bool g5, int compute
                               vec_prec, nrhs, in, out, active, n_active, s);
 }
 
+// FP64 stencil of points [p0, p1) on nsel listed sites (all when sel is null),
+// without the points whose bit is set in skip (per site, nullable): the hops
+// and the self term of the coarse-operator construction
+gmg_status coarse_apply_sel_f64(gmg_coarse* h, int p0, int p1, int nrhs, const double* in, double* out,
+                                const int32_t* sel, int nsel, const uint8_t* skip, cudaStream_t s) {
+  const LinkSel L{h->links_d.p, 9, 0, nullptr, h->nbr.as<int32_t>(), 0};
+  return coarse_mma<double>(L, in, out, (int)h->dims.vol(), h->N, nrhs, nullptr, nrhs, p0, p1, 0, sel, nsel, skip, s);
+}
+
 // ---------------------------------------------------------------------------
 // ConstructRemainingLinks (...DirsaveLut.h:1164-1196) / ForceHermitian
 // (CoarsenedMatrixUpstream.h:956-976) on the exchange layout:

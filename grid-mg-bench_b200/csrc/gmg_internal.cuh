@@ -125,7 +125,7 @@ struct gmg_agg {
   gmg::DevBuf scratch;
   gmg::DevBuf ortho_ws;  // orthonormalisation workspace (ortho.cu): status, per-block flags, Cholesky factors
   gmg::DevBuf dev_err;  // int: error code recorded by the tensor-core kernels
-  // CoarsenOperator workspace over the Wilson-clover operator (coarsen.cu),
+  // CoarsenOperator workspace (coarsen.cu),
   // kept between calls: fine fields of one batch of cw_nb basis vectors, the
   // projection output, per direction the fine sites of the backward faces
   // (global, cw_face) and their in-block indices (cw_sel), and per site the
@@ -178,6 +178,8 @@ gmg_status coarse_apply_simt(gmg_coarse* h, int p0, int p1, bool g5, int compute
 gmg_status coarse_apply_simt_ex(gmg_coarse* h, int src, int V, const int32_t* site_map, const int32_t* nbr,
                                 bool dag, int p0, int p1, bool g5, int compute, int vec_prec, int nrhs,
                                 const void* in, void* out, const int32_t* active, int n_active, cudaStream_t s);
+gmg_status coarse_apply_sel_f64(gmg_coarse* h, int p0, int p1, int nrhs, const double* in, double* out,
+                                const int32_t* sel, int nsel, const uint8_t* skip, cudaStream_t s);
 gmg_status coarse_construct_remaining(gmg_coarse* h, cudaStream_t s);
 
 // tensor-core multi-RHS stencil (coarse_mrhs_tc.cu)
