@@ -140,12 +140,27 @@ template <class Cx> struct ProjArgs {
   int N, dof, bv, nrhs;
   const int32_t* sel;
   int nsel;
+  // fine[site * fsite + r * frhs + k * fk].  face >= 0: a face field of the
+  // Wilson operator's hop `face` instead, sites c * nsel + s, with the upper two
+  // spins only; the lower two are (row of gamma, see face_spin) upper ones
+  int64_t fsite;
+  int frhs, fk, face;
   int units, rchunks, G, KS;
 };
 
 constexpr int kProjWarps = 8;
 
-template <class T, int MT, int RQ>
+// Lower spin s (2 or 3) of (1 -+ gamma_mu) psi is a phase (code 0: 1, 1: i, 2:
+// -1, 3: -i) times upper spin *from, for hop p (p < 4: +mu, the projector 1 -
+// gamma_mu; p >= 4: -mu, 1 + gamma_mu), in the gamma basis of the fine operator.
+__device__ __forceinline__ int face_spin(int p, int s, int* from) {
+  const int mu = p & 3;
+  *from = mu < 2 ? 3 - s : s - 2;
+  const int g = mu == 0 ? 3 : mu == 1 ? (s == 3 ? 2 : 0) : mu == 2 ? (s == 3 ? 1 : 3) : 0;
+  return (g + (p < 4 ? 2 : 0)) & 3;
+}
+
+template <class T, int MT, int RQ, bool FACE>
 __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const ProjArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -171,21 +186,26 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
 #pragma unroll
     for (int m = 0; m < MT; ++m) row[m] = min((mc * MT + m) * 8 + (lane >> 2), N - 1);
 #pragma unroll
-    for (int q = 0; q < RQ; ++q) foff[q] = min((rc * RQ + q) * 4 + (lane >> 3), a.nrhs - 1) * dof;
+    for (int q = 0; q < RQ; ++q) foff[q] = min((rc * RQ + q) * 4 + (lane >> 3), a.nrhs - 1) * a.frhs;
     const uint32_t s1 = f64mma::second_sign(part, true);
+    int from2 = 0, from3 = 0, code2 = 0, code3 = 0;
+    if (FACE) {
+      code2 = face_spin(a.face, 2, &from2);
+      code3 = face_spin(a.face, 3, &from3);
+    }
     Cx av[2][MT], fv[2][RQ];
-    int s = ks, k4 = 0, left = (nsites - ks + a.KS - 1) / a.KS * ((dof + 3) / 4);
+    int s = ks, k4 = 0, kc = kk, left = (nsites - ks + a.KS - 1) / a.KS * ((dof + 3) / 4);
     // the site requested next and the one after it
-    int sb = a.sel ? a.sel[s] : s, sf = blk[sb];
+    int sb = a.sel ? a.sel[s] : s, sf = FACE ? s : blk[sb];
     int sb1 = 0, sf1 = 0;
     const Cx *Vp, *Fp;
     auto at_site = [&]() {
       Vp = Vb + (int64_t)sb * dof;
-      Fp = a.fine + (int64_t)sf * a.nrhs * dof;
+      Fp = a.fine + (FACE ? c * a.nsel + sf : (int64_t)sf) * a.fsite;
       s += a.KS;
       if (s < nsites) {
         sb1 = a.sel ? a.sel[s] : s;
-        sf1 = blk[sb1];
+        sf1 = FACE ? s : blk[sb1];
       }
     };
     auto request = [&](Cx (&A)[MT], Cx (&F)[RQ]) {
@@ -194,7 +214,10 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
 #pragma unroll
       for (int m = 0; m < MT; ++m) A[m] = in_k ? __ldg(reinterpret_cast<const Cx*>(reinterpret_cast<const char*>(Vp + k) + (uint64_t)row[m] * Kb)) : Cx{0, 0};
 #pragma unroll
-      for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(Fp + foff[q] + k) : Cx{0, 0};
+      int kf = k;  // component stored for k
+      if (FACE && k >= 6) kf = k < 9 ? from2 * 3 + k - 6 : from3 * 3 + k - 9;
+#pragma unroll
+      for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(Fp + foff[q] + kf * a.fk) : Cx{0, 0};
       k4 += 4;
       if (k4 >= dof) {
         k4 = 0;
@@ -205,8 +228,20 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
     };
     auto multiply = [&](const Cx (&A)[MT], const Cx (&F)[RQ]) {
       double b0[RQ], b1[RQ];
+      if (FACE) {
+        // the phase as an exchange of the parts and signs of its own: i (x + i y) = -y + i x
+        const int code = kc < 6 ? 0 : kc < 9 ? code2 : code3;
+        const bool swap = code & 1;
+        const uint32_t neg = (code & 2) ? 0x80000000u : 0u;
+        const uint32_t nre = neg ^ (swap ? 0x80000000u : 0u);  // sign of the real part's source, of the imaginary's: neg
 #pragma unroll
-      for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, 0u, s1, b0[q], b1[q]);
+        for (int q = 0; q < RQ; ++q)
+          f64mma::expand(F[q], part ^ (swap ? 1 : 0), part ? neg : nre, (part ? nre : neg) ^ s1, b0[q], b1[q]);
+        kc = kc + 4 >= dof ? kk : kc + 4;
+      } else {
+#pragma unroll
+        for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, 0u, s1, b0[q], b1[q]);
+      }
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -265,9 +300,9 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
   }
 }
 
-template <class T, int MT, int RQ>
+template <class T, int MT, int RQ, bool FACE>
 static gmg_status launch_project(const ProjArgs<typename ctype<T>::t>& a, int Vc, cudaStream_t s) {
-  auto kern = project_mma_kernel<T, MT, RQ>;
+  auto kern = project_mma_kernel<T, MT, RQ, FACE>;
   const size_t smem = a.KS == 1 ? 0 : sizeof(double2) * 32 * MT * RQ * (size_t)a.G * a.KS;
   if (smem > 48 * 1024)
     GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -319,9 +354,12 @@ static ProjShape project_shape(int Vc, int MT, int mchunks, int rq) {
   return best;
 }
 
-template <class T>
-static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const void* fine, void* out, int64_t cstr,
-                              int64_t rstr, int64_t istr, const int32_t* sel, int nsel, cudaStream_t s) {
+// cmajor: fine is a component-major field [site][dof][nrhs] (else [site][nrhs][dof]);
+// FACE: a component-major field of the faces (see ProjArgs)
+template <class T, bool FACE = false>
+static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const void* fine, bool cmajor, int face,
+                              void* out, int64_t cstr, int64_t rstr, int64_t istr, const int32_t* sel, int nsel,
+                              cudaStream_t s) {
   typedef typename ctype<T>::t Cx;
   GMG_CHECK(sizeof(Cx) * 4 * h->dof * (size_t)(h->N + nrhs) <= 227 * 1024, GMG_ERR_UNSUPPORTED,
             "project: site dof x (nbasis + nrhs) too large");
@@ -331,15 +369,16 @@ static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const voi
   const ProjShape sh = project_shape(Vc, MT, mchunks, (nrhs + 3) / 4);
   const ProjArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
                        reinterpret_cast<const Cx*>(fine), reinterpret_cast<Cx*>(out), cstr, rstr, istr, h->N, h->dof,
-                       h->bv, nrhs, sel, nsel, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
+                       h->bv, nrhs, sel, nsel, (int64_t)nrhs * (FACE ? 6 : h->dof), cmajor ? 1 : h->dof,
+                       cmajor ? nrhs : 1, face, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
   auto by_rq = [&](auto mtc) -> gmg_status {
     constexpr int M = decltype(mtc)::value;
     switch (sh.w) {
-      case 1: return launch_project<T, M, 1>(a, Vc, s);
-      case 2: return launch_project<T, M, 2>(a, Vc, s);
-      case 3: return launch_project<T, M, 3>(a, Vc, s);
-      case 4: return launch_project<T, M, 4>(a, Vc, s);
-      default: return launch_project<T, M, 5>(a, Vc, s);
+      case 1: return launch_project<T, M, 1, FACE>(a, Vc, s);
+      case 2: return launch_project<T, M, 2, FACE>(a, Vc, s);
+      case 3: return launch_project<T, M, 3, FACE>(a, Vc, s);
+      case 4: return launch_project<T, M, 4, FACE>(a, Vc, s);
+      default: return launch_project<T, M, 5, FACE>(a, Vc, s);
     }
   };
   switch (MT) {
@@ -357,22 +396,25 @@ gmg_status agg_project(gmg_agg* h, int compute, int vec_prec, int nrhs, const vo
   GMG_CHECK(compute == vec_prec, GMG_ERR_UNSUPPORTED, "project: compute and vector precision differ");
   const int64_t N = h->N;
   if (compute == GMG_F64)
-    return project_mma<double>(h, h->basis_blk.p, nrhs, fine, coarse, nrhs * N, N, 1, nullptr, 0, s);
+    return project_mma<double>(h, h->basis_blk.p, nrhs, fine, false, -1, coarse, nrhs * N, N, 1, nullptr, 0, s);
   if (compute == GMG_F32) {
     GMG_TRY(agg_prepare_f32(h, s));
-    return project_mma<float>(h, h->basis_blk_f.p, nrhs, fine, coarse, nrhs * N, N, 1, nullptr, 0, s);
+    return project_mma<float>(h, h->basis_blk_f.p, nrhs, fine, false, -1, coarse, nrhs * N, N, 1, nullptr, 0, s);
   }
   return fail(GMG_ERR_UNSUPPORTED, "project: unsupported precision");
 }
 
 // FP64 projection over a subset of every block's sites (sel: nsel in-block
 // indices on the device, the same for all blocks; null: all of them), written
-// as columns i0 .. i0 + nrhs of the link matrices A[c][i][column]
-gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, double* A, int i0, const int32_t* sel, int nsel,
-                             cudaStream_t s) {
+// as columns i0 .. i0 + nrhs of the link matrices A[c][i][column].  face >= 0: of
+// the face field of the Wilson operator's hop `face` (wilson_face_half).
+gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, bool cmajor, int face, double* A, int i0,
+                             const int32_t* sel, int nsel, cudaStream_t s) {
   const int64_t N = h->N;
-  return project_mma<double>(h, h->basis_blk.p, nrhs, fine, reinterpret_cast<double2*>(A) + i0, N * N, 1, N, sel, nsel,
-                             s);
+  double2* out = reinterpret_cast<double2*>(A) + i0;
+  if (face >= 0)
+    return project_mma<double, true>(h, h->basis_blk.p, nrhs, fine, true, face, out, N * N, 1, N, sel, nsel, s);
+  return project_mma<double>(h, h->basis_blk.p, nrhs, fine, cmajor, -1, out, N * N, 1, N, sel, nsel, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -157,7 +157,6 @@ struct gmg_wilson {
   };
   std::map<int, PipePlan> pplans;
   gmg::DevBuf dev_err;    // device error word of the staged kernel
-  std::map<int, int> sel_pick;  // coarsening self term per nrhs: 0 pipelined staged kernel, 1 tile kernel
   int wforce = -1;                  // forced kernel variant (gmg_wilson_kernel), -1: autotuned
   std::map<uint64_t, int> wtune;    // autotuned variant per (precision, products, op class, nrhs class)
 };
@@ -199,8 +198,8 @@ gmg_status agg_basis_to_blocked(gmg_agg* h, const double* basis_dev, cudaStream_
 gmg_status agg_basis_from_blocked(gmg_agg* h, double* basis_dev, cudaStream_t s);
 gmg_status agg_project(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* fine,
                        void* coarse, cudaStream_t s);
-gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, double* A, int i0, const int32_t* sel, int nsel,
-                             cudaStream_t s);
+gmg_status agg_project_links(gmg_agg* h, int nrhs, const double* fine, bool cmajor, int face, double* A, int i0,
+                             const int32_t* sel, int nsel, cudaStream_t s);
 gmg_status agg_promote(gmg_agg* h, int compute, int vec_prec, int nrhs, const void* coarse,
                        void* fine, cudaStream_t s);
 // block orthonormalisation and its check (ortho.cu)
@@ -214,10 +213,11 @@ gmg_status agg_promote_tc(gmg_agg* h, int nrhs, const float* coarse, float* fine
 
 // fine Wilson-clover (wilson.cu)
 gmg_status wilson_build_clover(gmg_wilson* h, cudaStream_t s);
-gmg_status wilson_apply_face(gmg_wilson* h, int p, int nrhs, const double* in, double* out, const int32_t* sel,
-                             int nsel, cudaStream_t s);
-gmg_status wilson_apply_sel(gmg_wilson* h, int op, int dir, int disp, int nrhs, const double* in, double* out,
-                            const int32_t* sel, int nsel, const uint8_t* hskip, cudaStream_t s);
+// the coarsening's forms, on FP64 component-major fields [V][12][nrhs] (wilson.cu)
+gmg_status wilson_face_half(gmg_wilson* h, int p, int nrhs, const double* in, double* out, const int32_t* blk_sites,
+                            int64_t Vc, int bv, const int32_t* sel, int nsel, cudaStream_t s);
+gmg_status wilson_apply_masked(gmg_wilson* h, int nrhs, const double* in, double* out, const int32_t* sites,
+                               const uint8_t* hskip, cudaStream_t s);
 gmg_status wilson_apply(gmg_wilson* h, int op, int dir, int disp, int vec_prec, int nrhs,
                         const void* in, void* out, cudaStream_t s);
 gmg_status wilson_apply_mr(gmg_wilson* h, int vec_prec, int nrhs, const void* in, void* out, double2* d1,

@@ -319,10 +319,7 @@ __device__ __forceinline__ void st12x(typename wt<TO>::C* __restrict__ base, int
 }
 
 // DOTS (op M or MDAG): also add <out, in> and <out, out> of this (site, r) to
-// dsum[0..1] and dsum[2].  VEC: 16-byte spinor accesses.  skip: hops p with
-// bit p set are left out (0 for the plain operator); with the bits of the
-// hops to blocks of the other parity this gives e D e + o D o of the
-// coarsening's self term in one pass.
+// dsum[0..1] and dsum[2].  VEC: 16-byte spinor accesses.
 // VOUT: the output record layout (VEC by default); SUB: write bsub - M in
 // (bsub laid out and typed as the input) instead of M in.
 // NBS: nbr is a tile's staged neighbour table, entry p of this site at
@@ -333,7 +330,7 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
                                             const int32_t* __restrict__ nbr, const typename wt<TI>::C* __restrict__ in,
                                             typename wt<TO>::C* __restrict__ out, int V, int nrhs, int site, int r,
                                             T diag, int op, int dir, int disp, int apbc, int tvol, int Lt,
-                                            double* dsum = nullptr, int skip = 0,
+                                            double* dsum = nullptr,
                                             const typename wt<TI>::C* __restrict__ bsub = nullptr, int nbs_stride = 0,
                                             int nbs_i = 0) {
   typedef typename wt<T>::C C;
@@ -384,7 +381,6 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
       C cur[12];
       unraw12<T, TI>(cur, nxt);
       if (p < 7) ld12raw<T, TI, VEC>(nxt, in, nbs[p < 7 ? p + 1 : 7], r, nrhs);
-      if (skip & (1 << p)) continue;
       T coef = (T)-0.5;
       if (apbc && mu == 3 && ((dsp > 0 && tc == Lt - 1) || (dsp < 0 && tc == 0))) coef = (T)0.5;
       if (g5) {
@@ -420,7 +416,6 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
       const int mu = p & 3;
       const int dsp = p < 4 ? 1 : -1;
       if (op == GMG_OP_MDIR && (mu != dir || dsp != disp)) continue;
-      if (skip & (1 << p)) continue;
       const int nb = nbidx(p);
       T coef = (T)-0.5;
       if (apbc && mu == 3 && ((dsp > 0 && tc == Lt - 1) || (dsp < 0 && tc == 0))) coef = (T)0.5;
@@ -491,15 +486,10 @@ __global__ void __launch_bounds__(256) wilson_kernel(
 constexpr int kTileSites = 16;
 
 // bytes of one staging buffer of the tile kernel for link / clover entries of
-// csize bytes: the tile's hop links and clover blocks and, without SEL, its
-// neighbour table
-__host__ __device__ constexpr int tile_stage_bytes(int csize, bool sel) {
-  return csize * 2 * kTileSites * 72 + (sel ? 0 : 4 * 8 * kTileSites);
-}
+// csize bytes: the tile's hop links, clover blocks and neighbour table
+__host__ __device__ constexpr int tile_stage_bytes(int csize) { return csize * 2 * kTileSites * 72 + 4 * 8 * kTileSites; }
 // shared memory of a tile kernel launch (dots: the DOTS products' bytes)
-constexpr size_t tile_smem(int csize, bool sel, size_t dots) {
-  return (size_t)(sel ? 1 : 2) * tile_stage_bytes(csize, sel) + dots;
-}
+constexpr size_t tile_smem(int csize, size_t dots) { return (size_t)2 * tile_stage_bytes(csize) + dots; }
 
 // Multi-RHS tile kernel: a CTA takes kTileSites consecutive sites and all
 // right-hand sides (rt threads per site, each looping over its RHS); the
@@ -507,47 +497,40 @@ constexpr size_t tile_smem(int csize, bool sel, size_t dots) {
 // shared memory once and read by every RHS of the tile, the next tile's copied
 // (cp.async) into a second buffer while this one computes.  Thread per (site,
 // RHS) otherwise, spinors read from global memory.
-// SEL (the coarsening's self term, compiled separately): the tiles run over
-// the nsel sites of the list `sel` (all V sites when null) and only those are
-// written; hskip (per site, bit p: leave hop p out) restricts the hops to
-// neighbours of the same block parity (see wilson_site).
 // PF: the neighbour records are software-pipelined (see wilson_site).  (A
 // z-blocked tile order, as the staged kernel uses, measured no different here:
 // 2.73-2.79 ms at 32^4 x 24 RHS FP32 for z blocks of 1 to 32 planes.)
 // TI: the input vectors' precision (float with T = double: the FP64 operator
 // on FP32 vectors, promoted on load).
 // VOUT, SUB: the output layout and bsub - M in (see wilson_site).
-template <class T, bool DOTS, int MINB, bool SEL = false, int VEC = 1, bool PF = false, class TI = T, class TO = T,
+template <class T, bool DOTS, int MINB, int VEC = 1, bool PF = false, class TI = T, class TO = T,
           int VOUT = VEC, bool SUB = false>
 __global__ void __launch_bounds__(256, MINB) wilson_tile_kernel(
     const typename wt<T>::C* __restrict__ hop, const typename wt<T>::C* __restrict__ clover,
     const int32_t* __restrict__ nbr, const typename wt<TI>::C* __restrict__ in,
     typename wt<TO>::C* __restrict__ out, int V, int nrhs, int rt, T diag, int op, int dir, int disp,
     int apbc, int tvol, int Lt, double2* __restrict__ d1, double2* __restrict__ d2,
-    const int32_t* __restrict__ sel = nullptr, int nsel = 0, const uint8_t* __restrict__ hskip = nullptr,
     const typename wt<TI>::C* __restrict__ bsub = nullptr) {
   typedef typename wt<T>::C C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // staging buffers (tile_stage_bytes each; two without SEL, the next tile's
-  // filled while this one is computed): [kTileSites][8][9] hop links (p < 4
-  // U_mu(x), p >= 4 U_mu(x - mu)^dagger), [kTileSites][72] clover and, without
-  // SEL, the [8][kTileSites] neighbour table; then DOTS: [nrhs][3] products
-  constexpr int kBuf = tile_stage_bytes(sizeof(C), SEL);
-  double* Ds = reinterpret_cast<double*>(smem_raw + (SEL ? 1 : 2) * kBuf);
+  // two staging buffers (tile_stage_bytes each, the next tile's filled while
+  // this one is computed): [kTileSites][8][9] hop links (p < 4
+  // U_mu(x), p >= 4 U_mu(x - mu)^dagger), [kTileSites][72] clover and
+  // the [8][kTileSites] neighbour table; then DOTS: [nrhs][3] products
+  constexpr int kBuf = tile_stage_bytes(sizeof(C));
+  double* Ds = reinterpret_cast<double*>(smem_raw + 2 * kBuf);
   if (DOTS)
     for (int k = threadIdx.x; k < 3 * nrhs; k += blockDim.x) Ds[k] = 0.0;
-  const int nsites = (SEL && sel) ? nsel : V;
-  const int nt = (nsites + kTileSites - 1) / kTileSites;
+  const int nt = (V + kTileSites - 1) / kTileSites;
   const int sl = threadIdx.x / rt, rl = threadIdx.x % rt;
   const bool two = nrhs <= 2 * rt;
   double da[3] = {0.0, 0.0, 0.0}, db[3] = {0.0, 0.0, 0.0};
   // the tile's sites from buffer buf (links Ls, clover Cs, neighbour table Ns or nullptr)
   auto compute = [&](int tile, const C* Ls, const C* Cs, const int32_t* Ns) {
     const int s0 = tile * kTileSites;
-    const int ns = min(kTileSites, nsites - s0);
+    const int ns = min(kTileSites, V - s0);
     if (sl < ns) {
-      const int site = (SEL && sel) ? sel[s0 + sl] : s0 + sl;
-      const int skip = (SEL && hskip) ? hskip[site] : 0;
+      const int site = s0 + sl;
       const C* lsite = Ls + sl * 72;
       auto links = [&](int p, int) -> const C* { return lsite + p * 9; };
       // with two RHS or fewer per thread (rl, rl + rt) the thread owns them for
@@ -555,9 +538,9 @@ __global__ void __launch_bounds__(256, MINB) wilson_tile_kernel(
       int k = 0;
       for (int r = rl; r < nrhs; r += rt, ++k) {
         double dt[3] = {0.0, 0.0, 0.0};
-        wilson_site<T, decltype(links), DOTS, VEC, true, PF, TI, TO, VOUT, SUB, !SEL>(
-            Cs + sl * 72, links, SEL ? nbr : Ns, in, out, V, nrhs, site, r, diag, op, dir, disp, apbc, tvol, Lt, dt,
-            skip, bsub, kTileSites, sl);
+        wilson_site<T, decltype(links), DOTS, VEC, true, PF, TI, TO, VOUT, SUB, true>(
+            Cs + sl * 72, links, Ns, in, out, V, nrhs, site, r, diag, op, dir, disp, apbc, tvol, Lt, dt,
+            bsub, kTileSites, sl);
         if (DOTS) {
           if (two) {
 #pragma unroll
@@ -576,60 +559,43 @@ __global__ void __launch_bounds__(256, MINB) wilson_tile_kernel(
       }
     }
   };
-  if constexpr (SEL) {
-    C* Ls = reinterpret_cast<C*>(smem_raw);
-    C* Cs = Ls + kTileSites * 72;
-    for (int tile = blockIdx.x; tile < nt; tile += gridDim.x) {
+  // cp.async copies of a tile's links, clover (16-byte pieces: a site's 72
+  // entries are a multiple of 16 bytes, the arrays 16-byte aligned) and
+  // neighbour indices (4-byte pieces) into buffer b; one copy group per call,
+  // empty past the last tile
+  auto stage = [&](int tile, int b) {
+    if (tile < nt) {
       const int s0 = tile * kTileSites;
-      const int ns = min(kTileSites, nsites - s0);
-      __syncthreads();
-      for (int k = threadIdx.x; k < ns * 72; k += blockDim.x) {
-        const int64_t st = sel ? sel[s0 + k / 72] : s0 + k / 72;
-        Ls[k] = hop[st * 72 + k % 72];
-        Cs[k] = clover[st * 72 + k % 72];
+      const int ns = min(kTileSites, V - s0);
+      unsigned char* base = smem_raw + b * kBuf;
+      const int n16 = ns * 72 * (int)sizeof(C) / 16;
+      const unsigned char* hs = reinterpret_cast<const unsigned char*>(hop + (int64_t)s0 * 72);
+      const unsigned char* cs = reinterpret_cast<const unsigned char*>(clover + (int64_t)s0 * 72);
+      unsigned char* cd = base + kTileSites * 72 * sizeof(C);
+      for (int k = threadIdx.x; k < n16; k += blockDim.x) {
+        ac::cpa16(base + 16 * k, hs + 16 * k);
+        ac::cpa16(cd + 16 * k, cs + 16 * k);
       }
-      __syncthreads();
-      compute(tile, Ls, Cs, nullptr);
-    }
-  } else {
-    // cp.async copies of a tile's links, clover (16-byte pieces: a site's 72
-    // entries are a multiple of 16 bytes, the arrays 16-byte aligned) and
-    // neighbour indices (4-byte pieces) into buffer b; one copy group per call,
-    // empty past the last tile
-    auto stage = [&](int tile, int b) {
-      if (tile < nt) {
-        const int s0 = tile * kTileSites;
-        const int ns = min(kTileSites, nsites - s0);
-        unsigned char* base = smem_raw + b * kBuf;
-        const int n16 = ns * 72 * (int)sizeof(C) / 16;
-        const unsigned char* hs = reinterpret_cast<const unsigned char*>(hop + (int64_t)s0 * 72);
-        const unsigned char* cs = reinterpret_cast<const unsigned char*>(clover + (int64_t)s0 * 72);
-        unsigned char* cd = base + kTileSites * 72 * sizeof(C);
-        for (int k = threadIdx.x; k < n16; k += blockDim.x) {
-          ac::cpa16(base + 16 * k, hs + 16 * k);
-          ac::cpa16(cd + 16 * k, cs + 16 * k);
-        }
-        int32_t* nd = reinterpret_cast<int32_t*>(base + 2 * kTileSites * 72 * sizeof(C));
-        for (int k = threadIdx.x; k < 8 * ns; k += blockDim.x) {
-          const int p = k / ns, j = k - p * ns;
-          ac::cpa4(nd + p * kTileSites + j, nbr + (int64_t)p * V + s0 + j);
-        }
+      int32_t* nd = reinterpret_cast<int32_t*>(base + 2 * kTileSites * 72 * sizeof(C));
+      for (int k = threadIdx.x; k < 8 * ns; k += blockDim.x) {
+        const int p = k / ns, j = k - p * ns;
+        ac::cpa4(nd + p * kTileSites + j, nbr + (int64_t)p * V + s0 + j);
       }
-      ac::cpa_commit();
-    };
-    int b = 0;
-    stage(blockIdx.x, 0);
-    for (int tile = blockIdx.x; tile < nt; tile += gridDim.x, b ^= 1) {
-      stage(tile + gridDim.x, b ^ 1);  // buffer b ^ 1 was last read before the previous iteration's final barrier
-      ac::cpa_wait<1>();               // this thread's copies of this tile have landed
-      __syncthreads();                 // everyone's have
-      const unsigned char* base = smem_raw + b * kBuf;
-      const C* Ls = reinterpret_cast<const C*>(base);
-      compute(tile, Ls, Ls + kTileSites * 72, reinterpret_cast<const int32_t*>(base + 2 * kTileSites * 72 * sizeof(C)));
-      __syncthreads();  // buffer b is read: the next iteration's staging may overwrite it
     }
-    ac::cpa_wait<0>();
+    ac::cpa_commit();
+  };
+  int b = 0;
+  stage(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < nt; tile += gridDim.x, b ^= 1) {
+    stage(tile + gridDim.x, b ^ 1);  // buffer b ^ 1 was last read before the previous iteration's final barrier
+    ac::cpa_wait<1>();               // this thread's copies of this tile have landed
+    __syncthreads();                 // everyone's have
+    const unsigned char* base = smem_raw + b * kBuf;
+    const C* Ls = reinterpret_cast<const C*>(base);
+    compute(tile, Ls, Ls + kTileSites * 72, reinterpret_cast<const int32_t*>(base + 2 * kTileSites * 72 * sizeof(C)));
+    __syncthreads();  // buffer b is read: the next iteration's staging may overwrite it
   }
+  ac::cpa_wait<0>();
   if (DOTS) {
     if (two) {
 #pragma unroll
@@ -987,14 +953,13 @@ __device__ __forceinline__ void load_spinor(typename wt<T>::C* psi, const unsign
 }
 
 // the hop of direction MU of role h (p = 4 h + MU), unless left out
-template <class T, int MU, bool SKIP>
+template <class T, int MU>
 __device__ __forceinline__ void pipe_role_hop(typename wt<T>::C acc[4][3], const unsigned char* slots, int srec,
                                               const uint8_t* tab, const typename wt<T>::C* Ls, int rr, int h,
-                                              T sgn, bool g5, int op, int dir, int disp, int skipb, bool tedge,
+                                              T sgn, bool g5, int op, int dir, int disp, bool tedge,
                                               int apbc) {
   typedef typename wt<T>::C C;
   if (op == GMG_OP_MDIR && (MU != dir || disp != (h ? -1 : 1))) return;
-  if (SKIP && ((skipb >> (4 * h + MU)) & 1)) return;
   C psi[12];
   load_spinor<T>(psi, slots + tab[MU] * srec + rr * 12 * (int)sizeof(C), 12);
   if (g5) {
@@ -1005,12 +970,12 @@ __device__ __forceinline__ void pipe_role_hop(typename wt<T>::C acc[4][3], const
   pipe_hop<T, MU>(acc, Ls + (4 * h + MU) * 9, psi, sgn, coef);
 }
 
-template <class T, bool DOTS, bool SKIP>
+template <class T, bool DOTS>
 __global__ void __launch_bounds__(PipeGeo<T>::MAX_THREADS, 1) wilson_pipe_kernel(
     const typename wt<T>::C* __restrict__ hop, const typename wt<T>::C* __restrict__ clover,
     const PipeTile* __restrict__ tiles, const int32_t* __restrict__ tsites, const typename wt<T>::C* __restrict__ in,
     typename wt<T>::C* __restrict__ out, int nrhs, int ch, int nch, int ntiles, int nst, int ngrp, int sbytes, int soff,
-    T diag, int op, int dir, int disp, int apbc, int tvol, int Lt, const uint8_t* __restrict__ hskip,
+    T diag, int op, int dir, int disp, int apbc, int tvol, int Lt,
     double2* __restrict__ d1, double2* __restrict__ d2, int* __restrict__ err) {
   typedef typename wt<T>::C C;
   typedef PipeGeo<T> G;
@@ -1109,14 +1074,13 @@ __global__ void __launch_bounds__(PipeGeo<T>::MAX_THREADS, 1) wilson_pipe_kernel
       if (valid) {
         const int tc = site / tvol;
         const bool tedge = h ? tc == 0 : tc == Lt - 1;
-        const int skipb = SKIP ? (int)hskip[site] : 0;
         if (op != GMG_OP_MDIAG) {
           const uint8_t* tab = tp->slot + j * 8 + 4 * h;
           const C* Ls = reinterpret_cast<const C*>(sb + G::OFF_LINKS + j * G::LREC);
-          pipe_role_hop<T, 0, SKIP>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, skipb, tedge, apbc);
-          pipe_role_hop<T, 1, SKIP>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, skipb, tedge, apbc);
-          pipe_role_hop<T, 2, SKIP>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, skipb, tedge, apbc);
-          pipe_role_hop<T, 3, SKIP>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, skipb, tedge, apbc);
+          pipe_role_hop<T, 0>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, tedge, apbc);
+          pipe_role_hop<T, 1>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, tedge, apbc);
+          pipe_role_hop<T, 2>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, tedge, apbc);
+          pipe_role_hop<T, 3>(acc, slots, srec, tab, Ls, rr, h, sgn, g5, op, dir, disp, tedge, apbc);
         }
         if (op != GMG_OP_MDIR || DOTS) {
           // this role's chiral half of the site's own record (spins 2h, 2h + 1)
@@ -1433,12 +1397,10 @@ static int pipe_bz(const gmg_wilson* h, int64_t rec_bytes, double budget) {
 
 // pipelined staged kernel launch; *launched = false when it does not apply
 // (unaligned fields, no plan for this lattice, or too little shared memory for
-// two stages).  hskip (per site, bit p: leave hop p out) is the coarsening's
-// self-term restriction, or null.
+// two stages).
 template <bool DOTS>
 static gmg_status launch_pipe(gmg_wilson* h, int op, int dir, int disp, int vec_prec, int nrhs, const void* in,
-                              void* out, double2* d1, double2* d2, cudaStream_t s, bool* launched,
-                              const uint8_t* hskip = nullptr) {
+                              void* out, double2* d1, double2* d2, cudaStream_t s, bool* launched) {
   *launched = false;
   if (((uintptr_t)in | (uintptr_t)out) & 15) return GMG_OK;
   const bool f32 = vec_prec == GMG_F32;
@@ -1481,23 +1443,17 @@ static gmg_status launch_pipe(gmg_wilson* h, int op, int dir, int disp, int vec_
     GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<g, threads, smem, s>>>(reinterpret_cast<const C*>(hp), reinterpret_cast<const C*>(cp), tiles, tsites,
                                   reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), nrhs, ch, nch, ntiles,
-                                  nst, ngrp, sbytes, soff, diag, op, dir, disp, h->apbc, tvol, h->dims.d[3], hskip, d1, d2,
+                                  nst, ngrp, sbytes, soff, diag, op, dir, disp, h->apbc, tvol, h->dims.d[3], d1, d2,
                                   h->dev_err.as<int>());
     GMG_CUDA(cudaGetLastError());
     return GMG_OK;
   };
   if (f32) {
     const float diag = (float)(4.0 + h->mass);
-    if (hskip)
-      GMG_TRY(go(wilson_pipe_kernel<float, DOTS, true>, PipeCfg<float>::WARPS, diag, h->hop_f.p, h->clover_f.p));
-    else
-      GMG_TRY(go(wilson_pipe_kernel<float, DOTS, false>, PipeCfg<float>::WARPS, diag, h->hop_f.p, h->clover_f.p));
+    GMG_TRY(go(wilson_pipe_kernel<float, DOTS>, PipeCfg<float>::WARPS, diag, h->hop_f.p, h->clover_f.p));
   } else {
     const double diag = 4.0 + h->mass;
-    if (hskip)
-      GMG_TRY(go(wilson_pipe_kernel<double, DOTS, true>, PipeCfg<double>::WARPS, diag, h->hop.p, h->clover.p));
-    else
-      GMG_TRY(go(wilson_pipe_kernel<double, DOTS, false>, PipeCfg<double>::WARPS, diag, h->hop.p, h->clover.p));
+    GMG_TRY(go(wilson_pipe_kernel<double, DOTS>, PipeCfg<double>::WARPS, diag, h->hop.p, h->clover.p));
   }
   *launched = true;
   return GMG_OK;
@@ -1606,28 +1562,28 @@ static gmg_status launch_tile(gmg_wilson* h, int op, int dir, int disp, int vec_
   auto go = [&](auto kern, auto diag, const void* hp, const void* cp, size_t csize) -> gmg_status {
     typedef decltype(diag) T;
     typedef typename wt<T>::C C;
-    const size_t smem = tile_smem((int)csize, false, dots);
+    const size_t smem = tile_smem((int)csize, dots);
     if (smem > 48 * 1024) GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int g = wave_grid(kern, kTileSites * rt, smem, tiles);
     kern<<<g, kTileSites * rt, smem, s>>>(reinterpret_cast<const C*>(hp), reinterpret_cast<const C*>(cp),
                                           h->nbr.as<int32_t>(), reinterpret_cast<const C*>(in),
                                           reinterpret_cast<C*>(out), V, nrhs, rt, diag, op, dir, disp, h->apbc, tvol,
-                                          h->dims.d[3], d1, d2, nullptr, 0, nullptr, nullptr);
+                                          h->dims.d[3], d1, d2, nullptr);
     return GMG_OK;
   };
   if (vec_prec == GMG_F64) {
     const double diag = 4.0 + h->mass;
     if (v32)
-      GMG_TRY(go(wilson_tile_kernel<double, DOTS, 2, false, 2, true>, diag, h->hop.p, h->clover.p, sizeof(double2)));
+      GMG_TRY(go(wilson_tile_kernel<double, DOTS, 2, 2, true>, diag, h->hop.p, h->clover.p, sizeof(double2)));
     else
-      GMG_TRY(go(wilson_tile_kernel<double, DOTS, 2, false, 1>, diag, h->hop.p, h->clover.p, sizeof(double2)));
+      GMG_TRY(go(wilson_tile_kernel<double, DOTS, 2, 1>, diag, h->hop.p, h->clover.p, sizeof(double2)));
   } else if (vec_prec == GMG_F32) {
     const float diag = (float)(4.0 + h->mass);
     if (v32)
-      GMG_TRY(go(wilson_tile_kernel<float, DOTS, MINB, false, 2, PF>, diag, h->hop_f.p, h->clover_f.p,
+      GMG_TRY(go(wilson_tile_kernel<float, DOTS, MINB, 2, PF>, diag, h->hop_f.p, h->clover_f.p,
                  sizeof(float2)));
     else
-      GMG_TRY(go(wilson_tile_kernel<float, DOTS, MINB, false, 1>, diag, h->hop_f.p, h->clover_f.p, sizeof(float2)));
+      GMG_TRY(go(wilson_tile_kernel<float, DOTS, MINB, 1>, diag, h->hop_f.p, h->clover_f.p, sizeof(float2)));
   } else {
     return fail(GMG_ERR_UNSUPPORTED, "wilson apply: vectors must be F64 or F32");
   }
@@ -1751,207 +1707,221 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   return GMG_OK;
 }
 
-// Single-hop operator (Mdir of stencil point p) on a list of sites, FP64, for
-// the coarsening's face terms.  A CTA takes S = blockDim / nrhs sites: their
-// neighbour records (all RHS, 12 components each, contiguous in memory) come
-// into shared memory with coalesced loads, one thread per (site, RHS) applies
-// the hop from there into its own slot, and the results leave through the
-// same buffer with coalesced stores.  Slots are padded to 13 complex numbers so
-// that the 16-byte reads of consecutive RHS fall on different banks.  The
-// arithmetic is wilson_hop's, as in wilson_site with op GMG_OP_MDIR.
-constexpr int kFacePad = 13;
+// ---------------------------------------------------------------------------
+// The coarsening's forms of the FP64 operator, on component-major fields
+// [V][12][nrhs].  One warp's lanes hold consecutive right-hand sides of a site,
+// so a record load is 12 whole-line accesses (4 wavefronts each) instead of the
+// 32 partial lines per access of [V][nrhs][12] records at their 192-byte stride:
+// that L1 traffic and, in lattice order, the neighbours' second and third
+// trip from DRAM were the bound (32^4, 40 RHS: self term 12.15 ms, 47.7 GB).
+// ---------------------------------------------------------------------------
 
-template <int MU>
-__device__ __forceinline__ void face_hop(double2 acc[4][3], const double2* __restrict__ U, const double2* psi,
-                                         int disp, double coef) {
-  wilson_hop<double>(acc, U, false, psi, MU, disp, coef);  // backward links stored daggered
-}
-
-__global__ void __launch_bounds__(256, 3) wilson_face_hop_kernel(
+// Half of Mdir_p on nq listed in-block sites `sel` of every block: out[(c * nq +
+// q)][6][nrhs] = coef U (upper two spins of (1 -+ gamma_mu) psi(neighbour)).  The
+// lower two spins are fixed combinations of the upper ones, so the face
+// projections need these six components only (see project_half_kernel).
+__global__ void __launch_bounds__(256) wilson_face_half_kernel(
     const double2* __restrict__ hop, const int32_t* __restrict__ nbr, const double2* __restrict__ in,
-    double2* __restrict__ out, int V, int nrhs, const int32_t* __restrict__ sel, int nsel, int p, int apbc,
-    int tvol, int Lt) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int R = nrhs, W = nrhs * 12;
-  const int S = blockDim.x / R;
-  double2* rec = reinterpret_cast<double2*>(smem_raw);  // [S][R][kFacePad]
-  int* sidx = reinterpret_cast<int*>(rec + (size_t)S * R * kFacePad);
-  int* nidx = sidx + S;
-  const int mu = p & 3, disp = p < 4 ? 1 : -1;
-  const int t = threadIdx.x, q = t / R, r = t % R;
-  const int ntl = (nsel + S - 1) / S;
-  for (int tile = blockIdx.x; tile < ntl; tile += gridDim.x) {
-    const int s0 = tile * S, ns = min(S, nsel - s0);
-    __syncthreads();  // the previous tile's stores have read rec, sidx
-    if (t < ns) {
-      const int st = sel[s0 + t];
-      sidx[t] = st;
-      nidx[t] = nbr[(int64_t)p * V + st];
-    }
-    __syncthreads();
-    // one flat loop over the tile's records: its loads are independent and
-    // issue back to back (12 per thread for 40 RHS)
-#pragma unroll 12
-    for (int k = t; k < ns * W; k += blockDim.x) {
-      const int qq = k / W, e = k - qq * W;
-      rec[qq * R * kFacePad + (e / 12) * kFacePad + e % 12] = in[(int64_t)nidx[qq] * W + e];
-    }
-    __syncthreads();
-    if (q < ns) {
-      const int site = sidx[q];
-      double2* my = rec + (q * R + r) * kFacePad;
-      double2 psi[12];
+    double2* __restrict__ out, const int32_t* __restrict__ blk_sites, const int32_t* __restrict__ sel, int nq, int bv,
+    int64_t nfaces, int64_t V, int nrhs, int p, int apbc, int tvol, int Lt) {
+  const int mu = p & 3, disp = p < 4 ? 1 : -1, sgc = disp > 0 ? 2 : 0;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nfaces * nrhs;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t f = e / nrhs;
+    const int r = (int)(e - f * nrhs);
+    const int64_t c = f / nq;
+    const int site = blk_sites[c * bv + sel[f - c * nq]];
+    const double2* q = in + (int64_t)nbr[(int64_t)p * V + site] * 12 * nrhs + r;
+    double2 psi[12];
 #pragma unroll
-      for (int a = 0; a < 12; ++a) psi[a] = my[a];
-      double2 acc[4][3];
+    for (int k = 0; k < 12; ++k) psi[k] = __ldg(q + k * nrhs);
+    const int tc = site / tvol;
+    const double coef = apbc && mu == 3 && ((disp > 0 && tc == Lt - 1) || (disp < 0 && tc == 0)) ? 0.5 : -0.5;
+    const double2* U = hop + (int64_t)site * 72 + p * 9;
+    double2* o = out + f * 6 * nrhs + r;
+    auto body = [&](auto muc) {
+      constexpr int MU = decltype(muc)::value;
 #pragma unroll
-      for (int s2 = 0; s2 < 4; ++s2)
+      for (int s = 0; s < 2; ++s) {
+        const int code = (gphase(MU, s) + sgc) & 3;
+        double2 h[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[s2][c] = make_double2(0.0, 0.0);
-      const int tc = site / tvol;
-      double coef = -0.5;
-      if (apbc && mu == 3 && ((disp > 0 && tc == Lt - 1) || (disp < 0 && tc == 0))) coef = 0.5;
-      const double2* U = hop + (int64_t)site * 72 + p * 9;
-      switch (mu) {
-        case 0: face_hop<0>(acc, U, psi, disp, coef); break;
-        case 1: face_hop<1>(acc, U, psi, disp, coef); break;
-        case 2: face_hop<2>(acc, U, psi, disp, coef); break;
-        default: face_hop<3>(acc, U, psi, disp, coef); break;
-      }
+        for (int k = 0; k < 3; ++k) h[k] = cadd(psi[s * 3 + k], cphase(psi[gperm(MU, s) * 3 + k], code));
 #pragma unroll
-      for (int s2 = 0; s2 < 4; ++s2)
+        for (int a = 0; a < 3; ++a) {
+          double2 v{0.0, 0.0};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) my[s2 * 3 + c] = acc[s2][c];
-    }
-    __syncthreads();
-#pragma unroll 12
-    for (int k = t; k < ns * W; k += blockDim.x) {
-      const int qq = k / W, e = k - qq * W;
-      out[(int64_t)sidx[qq] * W + e] = rec[qq * R * kFacePad + (e / 12) * kFacePad + e % 12];
-    }
-  }
-}
-
-// out = Mdir_p in on the nsel sites of `sel` (FP64, nrhs <= 64); the other
-// sites of `out` are not written
-gmg_status wilson_apply_face(gmg_wilson* h, int p, int nrhs, const double* in, double* out, const int32_t* sel,
-                             int nsel, cudaStream_t s) {
-  GMG_CHECK(nrhs >= 1 && nrhs <= 64, GMG_ERR_UNSUPPORTED, "wilson face hop: nrhs must be in [1, 64]");
-  GMG_CHECK(p >= 0 && p < 8, GMG_ERR_ARGUMENT, "wilson face hop: bad stencil point");
-  if (nsel == 0) return GMG_OK;
-  const int V = (int)h->dims.vol();
-  const int tvol = h->dims.d[0] * h->dims.d[1] * h->dims.d[2];
-  const int S = std::max(1, 256 / nrhs);
-  const int threads = S * nrhs;
-  const size_t smem = sizeof(double2) * (size_t)S * nrhs * kFacePad + sizeof(int) * 2 * S;
-  if (smem > 48 * 1024)
-    GMG_CUDA(cudaFuncSetAttribute(wilson_face_hop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // all of the unified L1 / shared array as shared memory: three CTAs of
-  // 50 KB per SM, as many as the register bound allows (two with the default
-  // split)
-  GMG_CUDA(cudaFuncSetAttribute(wilson_face_hop_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  // one resident wave of CTAs looping over the tiles
-  int occ = 1, dev = 0, nsm = 148;
-  GMG_CUDA(cudaGetDevice(&dev));
-  GMG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  GMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wilson_face_hop_kernel, threads, smem));
-  const int tiles = (nsel + S - 1) / S;
-  const int g = std::min(tiles, nsm * std::max(occ, 1));
-  KernelTimer kt("wilson", s);
-  wilson_face_hop_kernel<<<g, threads, smem, s>>>(h->hop.as<double2>(), h->nbr.as<int32_t>(),
-                                                   reinterpret_cast<const double2*>(in),
-                                                   reinterpret_cast<double2*>(out), V, nrhs, sel, nsel, p, h->apbc,
-                                                   tvol, h->dims.d[3]);
-  GMG_CUDA(cudaGetLastError());
-  return GMG_OK;
-}
-
-// the tile kernel's SEL instance (FP64): op on the nsel sites of `sel` (all
-// sites when null), hops restricted by hskip; with all sites and 32-byte
-// aligned fields, 32-byte record accesses (the prefetching form spills here)
-static gmg_status launch_tile_sel(gmg_wilson* h, int op, int dir, int disp, int nrhs, const double* in, double* out,
-                                  const int32_t* sel, int nsel, const uint8_t* hskip, cudaStream_t s) {
-  const int V = (int)h->dims.vol();
-  const int tvol = h->dims.d[0] * h->dims.d[1] * h->dims.d[2];
-  int rt = 1;
-  for (int c = std::min(nrhs, 16); c >= 1; --c)
-    if (nrhs % c == 0) {
-      rt = c;
-      break;
-    }
-  if (nrhs > 16 && rt < 8) rt = 16;
-  const int nsites = sel ? nsel : V;
-  const int tiles = (nsites + kTileSites - 1) / kTileSites;
-  const int g = std::min(tiles, 148 * 16);
-  const size_t smem = tile_smem(sizeof(double2), true, 0);
-  const bool fast = !sel && ((((uintptr_t)in | (uintptr_t)out) & 31) == 0);
-  auto k = fast ? wilson_tile_kernel<double, false, 2, true, 2> : wilson_tile_kernel<double, false, 2, true>;
-  if (smem > 48 * 1024) GMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k<<<g, kTileSites * rt, smem, s>>>(h->hop.as<double2>(), h->clover.as<double2>(), h->nbr.as<int32_t>(),
-                                     (const double2*)in, (double2*)out, V, nrhs, rt, 4.0 + h->mass, op, dir, disp,
-                                     h->apbc, tvol, h->dims.d[3], nullptr, nullptr, sel, nsel, hskip, nullptr);
-  GMG_CUDA(cudaGetLastError());
-  return GMG_OK;
-}
-
-// The coarsening's forms of the FP64 operator: op on the nsel sites of `sel`
-// only (all sites when null; the other sites of `out` are not written), and
-// with hskip (per site, bit p set: leave hop p out) the hops restricted to
-// neighbours of the same block parity.  With all sites, the pipelined staged
-// kernel and the tile kernel are timed once per nrhs (not while the stream is
-// being captured) and the faster one is kept.
-gmg_status wilson_apply_sel(gmg_wilson* h, int op, int dir, int disp, int nrhs, const double* in, double* out,
-                            const int32_t* sel, int nsel, const uint8_t* hskip, cudaStream_t s) {
-  const int nsites = sel ? nsel : (int)h->dims.vol();
-  if (nsites == 0) return GMG_OK;
-  if (sel) {
-    KernelTimer kt("wilson", s);
-    return launch_tile_sel(h, op, dir, disp, nrhs, in, out, sel, nsel, hskip, s);
-  }
-  auto run = [&](int which, bool* launched) -> gmg_status {
-    if (which == 0)
-      return launch_pipe<false>(h, op, dir, disp, GMG_F64, nrhs, in, out, nullptr, nullptr, s, launched, hskip);
-    *launched = true;
-    return launch_tile_sel(h, op, dir, disp, nrhs, in, out, nullptr, 0, hskip, s);
-  };
-  int pick = 1;
-  auto it = h->sel_pick.find(nrhs);
-  if (it != h->sel_pick.end()) {
-    pick = it->second;
-  } else {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    GMG_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap == cudaStreamCaptureStatusNone) {
-      cudaEvent_t e0, e1;
-      GMG_CUDA(cudaEventCreate(&e0));
-      GMG_CUDA(cudaEventCreate(&e1));
-      float best = 1e30f;
-      gmg_status st = GMG_OK;
-      for (int which = 0; which < 2 && st == GMG_OK; ++which) {
-        bool launched = false;
-        st = run(which, &launched);  // warm-up
-        if (st != GMG_OK || !launched) continue;
-        if (cudaEventRecord(e0, s) != cudaSuccess) break;
-        for (int k = 0; k < 2 && st == GMG_OK; ++k) st = run(which, &launched);
-        float ms = 0.f;
-        if (st != GMG_OK || cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-            cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)
-          break;
-        if (ms < best) {
-          best = ms;
-          pick = which;
+          for (int b = 0; b < 3; ++b) v = cfma(__ldg(U + a * 3 + b), h[b], v);  // backward links stored daggered
+          o[(s * 3 + a) * nrhs] = make_double2(coef * v.x, coef * v.y);
         }
       }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      GMG_TRY(st);
-      if (best < 1e30f) h->sel_pick[nrhs] = pick;
+    };
+    switch (mu) {
+      case 0: body(std::integral_constant<int, 0>()); break;
+      case 1: body(std::integral_constant<int, 1>()); break;
+      case 2: body(std::integral_constant<int, 2>()); break;
+      default: body(std::integral_constant<int, 3>()); break;
     }
   }
+}
+
+gmg_status wilson_face_half(gmg_wilson* h, int p, int nrhs, const double* in, double* out, const int32_t* blk_sites,
+                            int64_t Vc, int bv, const int32_t* sel, int nsel, cudaStream_t s) {
+  const int64_t n = Vc * nsel * nrhs;
+  if (n == 0) return GMG_OK;
   KernelTimer kt("wilson", s);
-  bool launched = false;
-  GMG_TRY(run(pick, &launched));
-  if (!launched) GMG_TRY(run(1, &launched));
+  wilson_face_half_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 148 * 32), 256, 0, s>>>(
+      h->hop.as<double2>(), h->nbr.as<int32_t>(), reinterpret_cast<const double2*>(in),
+      reinterpret_cast<double2*>(out), blk_sites, sel, nsel, bv, Vc * nsel, h->dims.vol(), nrhs, p, h->apbc,
+      h->dims.d[0] * h->dims.d[1] * h->dims.d[2], h->dims.d[3]);
+  GMG_CUDA(cudaGetLastError());
+  return GMG_OK;
+}
+
+// out = M in without the hops whose bit is set in hskip (per site), the sites in
+// the order of the list `sites` (all V of them, block by block, so that a block's
+// neighbours come from L2 and, within a tile, from L1).  A CTA walks tiles of 16
+// sites, 8 lanes per site, a lane looping over its right-hand sides.  A site's 72
+// hop-link and 72 clover entries sit in shared memory at a stride of 145 complex
+// numbers (the four sites of a warp read distinct banks).  A hop's record is
+// requested before the previous hop's link multiply; the record is folded into
+// its half-spinor first, so that the requests reuse its registers.
+// What bounds it: the records' latency at the occupancy its registers leave (3
+// CTAs per SM).  One staging buffer, not two: the shared memory of a second one
+// (74 KB per CTA) takes the L1 that holds a tile's records between its sites'
+// hops (L1 hit rate 4 %, 9.4 ms; with one 5.85 ms; 4 CTAs per SM, spilling: 9.2;
+// two threads per record, one per pair of spins, at 24 warps per SM: 10.2).
+// 32^4, 40 RHS: 12.15 ms (47.7 GB from DRAM) -> 5.85 ms.
+constexpr int kMaskSites = 16, kMaskLanes = 8, kMaskStride = 145;
+__device__ __forceinline__ double2 zfma(double2 a, double2 b, double2 acc) {
+  acc.x = fma(a.x, b.x, acc.x);
+  acc.x = fma(-a.y, b.y, acc.x);
+  acc.y = fma(a.x, b.y, acc.y);
+  acc.y = fma(a.y, b.x, acc.y);
+  return acc;
+}
+
+__global__ void __launch_bounds__(kMaskSites* kMaskLanes, 3) wilson_masked_kernel(
+    const double2* __restrict__ hop, const double2* __restrict__ clover, const int32_t* __restrict__ nbr,
+    const double2* __restrict__ in, double2* __restrict__ out, const int32_t* __restrict__ sites,
+    const uint8_t* __restrict__ hskip, int V, int nrhs, double diag, int apbc, int tvol, int Lt) {
+  extern __shared__ __align__(16) double2 msm[];  // [kMaskSites][kMaskStride], then two tables
+  int* tab = reinterpret_cast<int*>(msm + kMaskSites * kMaskStride);  // [2][10][kMaskSites]: 8 neighbours, site, skip
+  const int t = threadIdx.x, sl = t / kMaskLanes, rl = t % kMaskLanes;
+  const int nt = (V + kMaskSites - 1) / kMaskSites;
+  // this thread's table entries of a tile: neighbour p = t / 16 of site t % 16, and its site and skip mask (p = 0)
+  static_assert(kMaskSites * kMaskLanes == 8 * kMaskSites, "one neighbour entry per thread");
+  auto entry = [&](int tile, int& nb, int& st, int& sk) {
+    const int e = tile * kMaskSites + t % kMaskSites;
+    nb = st = sk = 0;
+    if (tile < nt && e < V) {
+      st = sites[e];
+      nb = nbr[(int64_t)(t / kMaskSites) * V + st];
+      sk = hskip[st];
+    }
+  };
+  auto put = [&](int b, int nb, int st, int sk) {
+    int* d = tab + b * 10 * kMaskSites + t % kMaskSites;
+    d[t / kMaskSites * kMaskSites] = nb;
+    if (t < kMaskSites) {
+      d[8 * kMaskSites] = st;
+      d[9 * kMaskSites] = sk;
+    }
+  };
+  int nb, st, sk, b = 0;
+  entry(blockIdx.x, nb, st, sk);
+  put(0, nb, st, sk);
+  for (int tile = blockIdx.x; tile < nt; tile += gridDim.x, b ^= 1) {
+    const int ns = min(kMaskSites, V - tile * kMaskSites);
+    double2* Us = msm + sl * kMaskStride;
+    if (sl < ns) {
+      const int64_t here = sites[tile * kMaskSites + sl];
+      const double2 *hs = hop + here * 72, *cs = clover + here * 72;
+#pragma unroll
+      for (int k = rl; k < 72; k += kMaskLanes) {
+        ac::cpa16(Us + k, hs + k);
+        ac::cpa16(Us + 72 + k, cs + k);
+      }
+    }
+    ac::cpa_commit();
+    entry(tile + gridDim.x, nb, st, sk);
+    ac::cpa_wait<0>();
+    __syncthreads();
+    if (sl < ns) {
+      const double2* Cs = Us + 72;
+      const int* T = tab + b * 10 * kMaskSites + sl;
+      const int site = T[8 * kMaskSites], skip = T[9 * kMaskSites], tc = site / tvol;
+      for (int r = rl; r < nrhs; r += kMaskLanes) {
+        double2 cur[12], acc[12];
+        auto request = [&](int s) {
+          const double2* q = in + (int64_t)s * 12 * nrhs + r;
+#pragma unroll
+          for (int k = 0; k < 12; ++k) cur[k] = __ldg(q + k * nrhs);
+        };
+        request(site);
+#pragma unroll
+        for (int a = 0; a < 12; ++a) {
+          double2 v = make_double2(diag * cur[a].x, diag * cur[a].y);
+#pragma unroll
+          for (int q = 0; q < 6; ++q) v = zfma(Cs[a * 6 + q], cur[a / 6 * 6 + q], v);
+          acc[a] = v;
+        }
+        if (!(skip & 1)) request(T[0]);
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+          const int mu = p & 3, sgc = p < 4 ? 2 : 0;
+          const bool on = !(skip & (1 << p));
+          double2 h[6];
+          if (on) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+#pragma unroll
+              for (int k = 0; k < 3; ++k)
+                h[s * 3 + k] = cadd(cur[s * 3 + k], cphase(cur[gperm(mu, s) * 3 + k], (gphase(mu, s) + sgc) & 3));
+          }
+          if (p < 7 && !(skip & (2 << p))) request(T[(p + 1) * kMaskSites]);
+          if (on) {
+            const double coef = apbc && mu == 3 && tc == (p < 4 ? Lt - 1 : 0) ? 0.5 : -0.5;
+            const double2* U = Us + p * 9;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+              double2 uh[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll
+              for (int k = 0; k < 3; ++k) {
+                const double2 u = U[a * 3 + k];
+                uh[0] = zfma(u, h[k], uh[0]);
+                uh[1] = zfma(u, h[3 + k], uh[1]);
+              }
+#pragma unroll
+              for (int s = 0; s < 4; ++s) {
+                const double2 v = s < 2 ? uh[s] : cphase(uh[gperm(mu, s)], (gphase(mu, s) + sgc) & 3);
+                acc[s * 3 + a].x = fma(coef, v.x, acc[s * 3 + a].x);
+                acc[s * 3 + a].y = fma(coef, v.y, acc[s * 3 + a].y);
+              }
+            }
+          }
+        }
+        double2* o = out + (int64_t)site * 12 * nrhs + r;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) o[k * nrhs] = acc[k];
+      }
+    }
+    put(b ^ 1, nb, st, sk);
+    __syncthreads();
+  }
+}
+
+gmg_status wilson_apply_masked(gmg_wilson* h, int nrhs, const double* in, double* out, const int32_t* sites,
+                               const uint8_t* hskip, cudaStream_t s) {
+  const int V = (int)h->dims.vol();
+  const size_t smem = sizeof(double2) * kMaskSites * kMaskStride + sizeof(int) * 2 * 10 * kMaskSites;
+  GMG_CUDA(cudaFuncSetAttribute(wilson_masked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  KernelTimer kt("wilson", s);
+  wilson_masked_kernel<<<std::min((V + kMaskSites - 1) / kMaskSites, 148 * 3), kMaskSites * kMaskLanes, smem, s>>>(
+      h->hop.as<double2>(), h->clover.as<double2>(), h->nbr.as<int32_t>(), reinterpret_cast<const double2*>(in),
+      reinterpret_cast<double2*>(out), sites, hskip, V, nrhs, 4.0 + h->mass, h->apbc,
+      h->dims.d[0] * h->dims.d[1] * h->dims.d[2], h->dims.d[3]);
+  GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
 
@@ -1975,7 +1945,7 @@ gmg_status wilson_apply_f32_in(gmg_wilson* h, int op, int nrhs, const float* in,
   if (nrhs > 16 && rt < 8) rt = 16;
   const int tiles = (V + kTileSites - 1) / kTileSites;
   const int g = std::min(tiles, 148 * 16);
-  const size_t smem = tile_smem(sizeof(double2), false, 0);
+  const size_t smem = tile_smem(sizeof(double2), 0);
   const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
   KernelTimer kt("wilson", s);
   auto go = [&](auto kern) -> gmg_status {
@@ -1984,13 +1954,13 @@ gmg_status wilson_apply_f32_in(gmg_wilson* h, int op, int nrhs, const float* in,
     kern<<<g, kTileSites * rt, smem, s>>>(h->hop.as<double2>(), h->clover.as<double2>(), h->nbr.as<int32_t>(),
                                           reinterpret_cast<const float2*>(in), reinterpret_cast<double2*>(out), V,
                                           nrhs, rt, 4.0 + h->mass, op, 0, 0, h->apbc, tvol, h->dims.d[3], nullptr,
-                                          nullptr, nullptr, 0, nullptr, nullptr);
+                                          nullptr, nullptr);
     GMG_CUDA(cudaGetLastError());
     return GMG_OK;
   };
-  if ((al & 31) == 0) return go(wilson_tile_kernel<double, false, 2, false, 2, true, float>);
-  if ((al & 15) == 0) return go(wilson_tile_kernel<double, false, 2, false, 1, true, float>);
-  return go(wilson_tile_kernel<double, false, 2, false, 0, true, float>);
+  if ((al & 31) == 0) return go(wilson_tile_kernel<double, false, 2, 2, true, float>);
+  if ((al & 15) == 0) return go(wilson_tile_kernel<double, false, 2, 1, true, float>);
+  return go(wilson_tile_kernel<double, false, 2, 0, true, float>);
 }
 
 // out = M in with the minimal-residual inner products d1[r] = <out, in>,
@@ -2016,17 +1986,17 @@ gmg_status wilson_apply_mr_bf16(gmg_wilson* h, int nrhs, const uint32_t* in, uin
   if (nrhs > 16 && rt < 8) rt = 16;
   const int tiles = (V + kTileSites - 1) / kTileSites;
 
-  const size_t smem = tile_smem(sizeof(float2), false, sizeof(double) * 3 * (size_t)nrhs);
+  const size_t smem = tile_smem(sizeof(float2), sizeof(double) * 3 * (size_t)nrhs);
   KernelTimer kt("wilson", s);
   GMG_CUDA(cudaMemsetAsync(d1, 0, sizeof(double2) * nrhs, s));
   GMG_CUDA(cudaMemsetAsync(d2, 0, sizeof(double2) * nrhs, s));
-  auto k = blocked ? wilson_tile_kernel<float, true, 3, false, 3, true, bf16s, bf16s>
-                   : wilson_tile_kernel<float, true, 3, false, 1, true, bf16s, bf16s>;
+  auto k = blocked ? wilson_tile_kernel<float, true, 3, 3, true, bf16s, bf16s>
+                   : wilson_tile_kernel<float, true, 3, 1, true, bf16s, bf16s>;
   if (smem > 48 * 1024) GMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int g = wave_grid(k, kTileSites * rt, smem, tiles);
   k<<<g, kTileSites * rt, smem, s>>>(h->hop_f.as<float2>(), h->clover_f.as<float2>(), h->nbr.as<int32_t>(), in, out, V,
                                      nrhs, rt, (float)(4.0 + h->mass), GMG_OP_M, 0, 0, h->apbc, tvol, h->dims.d[3], d1,
-                                     d2, nullptr, 0, nullptr, nullptr);
+                                     d2, nullptr);
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
@@ -2051,15 +2021,15 @@ gmg_status wilson_residual_bf16(gmg_wilson* h, int nrhs, const float* b, const f
     }
   if (nrhs > 16 && rt < 8) rt = 16;
   const int tiles = (V + kTileSites - 1) / kTileSites;
-  const size_t smem = tile_smem(sizeof(float2), false, 0);
+  const size_t smem = tile_smem(sizeof(float2), 0);
   KernelTimer kt("wilson", s);
-  auto k = wilson_tile_kernel<float, false, 3, false, 2, true, float, bf16s, 3, true>;
+  auto k = wilson_tile_kernel<float, false, 3, 2, true, float, bf16s, 3, true>;
   if (smem > 48 * 1024) GMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int g = wave_grid(k, kTileSites * rt, smem, tiles);
   k<<<g, kTileSites * rt, smem, s>>>(h->hop_f.as<float2>(), h->clover_f.as<float2>(), h->nbr.as<int32_t>(),
                                      reinterpret_cast<const float2*>(x), out, V, nrhs, rt, (float)(4.0 + h->mass),
-                                     GMG_OP_M, 0, 0, h->apbc, tvol, h->dims.d[3], nullptr, nullptr, nullptr, 0,
-                                     nullptr, reinterpret_cast<const float2*>(b));
+                                     GMG_OP_M, 0, 0, h->apbc, tvol, h->dims.d[3], nullptr, nullptr,
+                                     reinterpret_cast<const float2*>(b));
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
@@ -2080,15 +2050,15 @@ gmg_status wilson_residual_f64(gmg_wilson* h, int nrhs, const double* b, const d
     }
   if (nrhs > 16 && rt < 8) rt = 16;
   const int tiles = (V + kTileSites - 1) / kTileSites;
-  const size_t smem = tile_smem(sizeof(double2), false, 0);
+  const size_t smem = tile_smem(sizeof(double2), 0);
   KernelTimer kt("wilson", s);
-  auto k = wilson_tile_kernel<double, false, 2, false, 2, true, double, double, 2, true>;
+  auto k = wilson_tile_kernel<double, false, 2, 2, true, double, double, 2, true>;
   if (smem > 48 * 1024) GMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int g = wave_grid(k, kTileSites * rt, smem, tiles);
   k<<<g, kTileSites * rt, smem, s>>>(h->hop.as<double2>(), h->clover.as<double2>(), h->nbr.as<int32_t>(),
                                      reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(r), V, nrhs, rt,
                                      4.0 + h->mass, GMG_OP_M, 0, 0, h->apbc, tvol, h->dims.d[3], nullptr, nullptr,
-                                     nullptr, 0, nullptr, reinterpret_cast<const double2*>(b));
+                                     reinterpret_cast<const double2*>(b));
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }

@@ -98,3 +98,42 @@ def test_project_and_promote(fd, cd, dof, N, R, dt):
     ag.PromoteFromSubspace(_dev(c, dt), got_f)
     assert orc.rel_dev_sq(orc.block_project(fd, cd, B, f), _host(got_c)) < TOL[dt]
     assert orc.rel_dev_sq(orc.block_promote(fd, cd, B, c), _host(got_f)) < TOL[dt]
+
+
+@pytest.mark.parametrize("fd,cd,nvec,batch", [
+    ((6, 4, 4, 6), (2, 2, 2, 2), 5, 0),   # block sizes 3 and 2, nbasis 10
+    ((6, 4, 6, 4), (3, 2, 3, 1), 3, 4),   # odd coarse extents and one of 1, batches of 4 and 2
+    ((4, 6, 4, 4), (4, 3, 2, 2), 9, 0),   # block extent 1: every site on a face; 144 sites, nbasis 18
+])
+def test_coarsen_wilson_edges(fd, cd, nvec, batch):
+    U = inputs.hot_gauge(fd, inputs.rng(stream=730 + nvec))
+    h = inputs.gaussian_field((nvec, int(np.prod(fd)), 12), inputs.rng(stream=740 + nvec))
+    B = orc.chiral_double(h, 0.5)
+    ag = gmg.Aggregation(fd, cd, 12, 2 * nvec)
+    ag.set_basis(B)
+    ag.set_coarsen_batch(batch)
+    w = gmg.WilsonClover(fd, -0.1, 1.0, antiperiodic=1)
+    w.set_gauge(U)
+    cm = gmg.CoarsenedMatrix(cd, 2 * nvec)
+    cm.CoarsenOperator(ag, w)
+    ref = orc.coarsen_wilson(fd, cd, B, U, orc.clover_build(fd, U, 1.0), -0.1, 1, 0, variant=1)
+    got = cm.get_links()
+    for p in range(9):
+        assert orc.rel_dev_sq(ref[p], got[p]) < 1e-15, p
+
+
+def test_coarsen_coarse_edges():
+    fd, cd, dof, nvec = (6, 4, 4, 2), (3, 2, 2, 1), 10, 4  # odd coarse extents, site dof not a multiple of 4
+    r = inputs.rng(stream=750)
+    A = inputs.random_links(fd, dof, r)
+    B = orc.chiral_double(inputs.gaussian_field((nvec, int(np.prod(fd)), dof), r), 0.5)
+    fine = gmg.CoarsenedMatrix(fd, dof)
+    fine.set_links(A)
+    ag = gmg.Aggregation(fd, cd, dof, 2 * nvec)
+    ag.set_basis(B)
+    cm = gmg.CoarsenedMatrix(cd, 2 * nvec)
+    cm.CoarsenOperator(ag, fine)
+    ref = orc.coarsen_coarse(fd, cd, B, A, variant=1)
+    got = cm.get_links()
+    for p in range(9):
+        assert orc.rel_dev_sq(ref[p], got[p]) < 1e-15, p
