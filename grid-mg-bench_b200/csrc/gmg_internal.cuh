@@ -146,6 +146,9 @@ struct gmg_wilson {
   gmg::DevBuf clover;     // complex<double> [V][2][6][6]
   gmg::DevBuf clover_f;
   gmg::DevBuf nbr;        // int32 [9][V]
+  // the site kernel's copies of links and clover, [V / 32][36][32] (wilson.cu)
+  gmg::DevBuf soa_gauge, soa_gauge_f, soa_clover, soa_clover_f;
+  bool soa_ok = false, soa_f_ok = false;
   // hop links [V][8][3][3] (p < 4: U_mu(x), p >= 4: U_mu(x - mu)^dagger) for
   // the tile, staged and face-hop kernels
   gmg::DevBuf hop, hop_f;

@@ -462,25 +462,113 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
   }
 }
 
-// thread per (site, rhs); links and clover read from global memory (few RHS)
-template <class T>
-__global__ void __launch_bounds__(256) wilson_kernel(
+// Thread per (site, rhs), for few right-hand sides: with one or two uses per link
+// the operator is bound by its bytes, so the lanes of a warp, which hold
+// consecutive sites, read the links and the clover from copies in which the same
+// entry of 32 consecutive sites lies in one run ([V / 32][36][32]), and the clover
+// as 36 complex numbers per site instead of 72 (its two blocks are Hermitian to the
+// last bit: per block 3 pairs of diagonal values, then the 15 entries above them).
+// The backward hops read U_mu(x - mu) of the neighbour's run.  Per site and RHS
+// that is 1536 bytes in FP64, against 2112 for the site-major arrays, whose
+// 16-byte reads at 576- and 1152-byte strides also took a line each.  32^4, one
+// RHS: FP64 847 -> 380 us (1.6 GB, 4.2 TB/s; 390 and 575 us at 4 and 5 CTAs per SM,
+// which spill), FP32 497 -> 168 us (189 at 4 CTAs per SM).
+constexpr int kSoa = 32, kSoaThreads = 128;
+
+template <class C>
+__global__ void soa_kernel(const C* __restrict__ gauge, const C* __restrict__ clover, C* __restrict__ g,
+                           C* __restrict__ c, int64_t V) {
+  const int64_t total = (V + kSoa - 1) / kSoa * kSoa * 36;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = (int)(e % kSoa), k = (int)(e / kSoa % 36);
+    const int64_t site = e / (36 * kSoa) * kSoa + lane;
+    if (site >= V) continue;
+    g[e] = gauge[site * 36 + k];
+    const int blk = k / 18, q = k % 18;
+    const C* m = clover + site * 72 + blk * 36;
+    if (q < 3) {
+      c[e] = C{m[2 * q * 7].x, m[(2 * q + 1) * 7].x};
+    } else {
+      int a = 0, n = q - 3;  // entry n of the rows above the diagonal: row a, column a + 1 + n
+      while (n >= 5 - a) n -= 5 - a++;
+      c[e] = m[a * 6 + a + 1 + n];
+    }
+  }
+}
+
+template <class T, int VEC>
+__global__ void __launch_bounds__(kSoaThreads, sizeof(T) == 8 ? 3 : 6) wilson_kernel(
     const typename wt<T>::C* __restrict__ gauge, const typename wt<T>::C* __restrict__ clover,
     const int32_t* __restrict__ nbr, const typename wt<T>::C* __restrict__ in,
     typename wt<T>::C* __restrict__ out, int V, int nrhs, T diag, int op, int dir, int disp,
     int apbc, int tvol, int Lt) {
   typedef typename wt<T>::C C;
-  const int64_t total = (int64_t)V * nrhs;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int site = (int)(e / nrhs);
-    const int r = (int)(e % nrhs);
-    auto links = [&](int p, int nb) -> const C* {
-      return gauge + ((int64_t)(p < 4 ? site : nb) * 4 + (p & 3)) * 9;
-    };
-    wilson_site<T>(clover + (int64_t)site * 72, links, nbr, in, out, V, nrhs, site, r, diag, op, dir, disp, apbc, tvol,
-                   Lt);
+  const int r = blockIdx.x % nrhs;  // the right-hand sides of a run of sites next to one another: links from L2
+  const int site = (int)(blockIdx.x / nrhs) * kSoaThreads + threadIdx.x;
+  if (site >= V) return;
+  const bool g5 = op == GMG_OP_MDAG;
+  const int tc = site / tvol;
+  auto record = [&](C (&psi)[12], int s) {
+    ld12x<T, T, VEC>(psi, in, s, r, nrhs);
+#pragma unroll
+    for (int k = 6; k < 12; ++k)
+      if (g5) psi[k] = C{-psi[k].x, -psi[k].y};
+  };
+  C acc[4][3];
+  if (op != GMG_OP_MDIR) {
+    C psi[12], v[12];
+    record(psi, site);
+    const C* c = clover + (int64_t)(site / kSoa) * 36 * kSoa + site % kSoa;
+#pragma unroll
+    for (int blk = 0; blk < 2; ++blk) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const C d = __ldg(c + (blk * 18 + q) * kSoa);
+        const int a = blk * 6 + 2 * q;
+        v[a] = C{(diag + d.x) * psi[a].x, (diag + d.x) * psi[a].y};
+        v[a + 1] = C{(diag + d.y) * psi[a + 1].x, (diag + d.y) * psi[a + 1].y};
+      }
+      int k = blk * 18 + 3;
+#pragma unroll
+      for (int a = 0; a < 6; ++a)
+#pragma unroll
+        for (int b = a + 1; b < 6; ++b, ++k) {
+          const C m = __ldg(c + k * kSoa);
+          v[blk * 6 + a] = cfma(m, psi[blk * 6 + b], v[blk * 6 + a]);
+          v[blk * 6 + b] = cfmac(m, psi[blk * 6 + a], v[blk * 6 + b]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k / 3][k % 3] = v[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k / 3][k % 3] = C{0, 0};
   }
+  if (op != GMG_OP_MDIAG) {
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const int mu = p & 3, dsp = p < 4 ? 1 : -1;
+      if (op == GMG_OP_MDIR && (mu != dir || dsp != disp)) continue;
+      const int nb = nbr[(int64_t)p * V + site];
+      T coef = (T)-0.5;
+      if (apbc && mu == 3 && tc == (dsp > 0 ? Lt - 1 : 0)) coef = (T)0.5;
+      const int ls = dsp > 0 ? site : nb;
+      const C* g = gauge + ((int64_t)(ls / kSoa) * 36 + mu * 9) * kSoa + ls % kSoa;
+      C U[9], psi[12];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) U[k] = __ldg(g + k * kSoa);
+      record(psi, nb);
+      wilson_hop<T>(acc, U, dsp < 0, psi, mu, dsp, coef);
+    }
+  }
+  C ov[12];
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    ov[k] = acc[k / 3][k % 3];
+    if (g5 && k >= 6) ov[k] = C{-ov[k].x, -ov[k].y};
+  }
+  st12x<T, T, VEC>(out, site, r, nrhs, ov);
 }
 
 constexpr int kTileSites = 16;
@@ -1290,6 +1378,7 @@ __global__ void d2f_wilson(const double2* __restrict__ a, float2* __restrict__ b
 
 gmg_status wilson_build_clover(gmg_wilson* h, cudaStream_t s) {
   const int V = (int)h->dims.vol();
+  h->soa_ok = h->soa_f_ok = false;
   GMG_TRY(h->clover.alloc(sizeof(double2) * 72 * (size_t)V));
   GMG_TRY(h->clover_f.alloc(sizeof(float2) * 72 * (size_t)V));
   GMG_TRY(h->gauge_f.alloc(sizeof(float2) * 36 * (size_t)V));
@@ -1501,27 +1590,63 @@ static gmg_status launch_quad(gmg_wilson* h, int op, int dir, int disp, int vec_
 }
 
 // thread per (site, RHS), links and clover from global memory
-static gmg_status launch_site(gmg_wilson* h, int op, int dir, int disp, int vec_prec, int nrhs, const void* in,
-                              void* out, cudaStream_t s) {
-  const int V = (int)h->dims.vol();
-  const int tvol = h->dims.d[0] * h->dims.d[1] * h->dims.d[2];
-  const int64_t total = (int64_t)V * nrhs;
-  const int grid = (int)std::min<int64_t>((total + 127) / 128, 148 * 32);
-  if (vec_prec == GMG_F64) {
-    wilson_kernel<double><<<grid, 128, 0, s>>>(h->gauge.as<double2>(), h->clover.as<double2>(),
-                                                h->nbr.as<int32_t>(), (const double2*)in, (double2*)out, V,
-                                                nrhs, 4.0 + h->mass, op, dir, disp, h->apbc, tvol,
-                                                h->dims.d[3]);
-  } else if (vec_prec == GMG_F32) {
-    wilson_kernel<float><<<grid, 128, 0, s>>>(h->gauge_f.as<float2>(), h->clover_f.as<float2>(),
-                                               h->nbr.as<int32_t>(), (const float2*)in, (float2*)out, V,
-                                               nrhs, (float)(4.0 + h->mass), op, dir, disp, h->apbc, tvol,
-                                               h->dims.d[3]);
-  } else {
-    return fail(GMG_ERR_UNSUPPORTED, "wilson apply: vectors must be F64 or F32");
+// The site kernel's copies of the links and the clover in precision f64 / f32, built
+// on the first launch that finds none (not while the stream is being captured, nor
+// when the device memory does not suffice: *ok = false).  Other streams may use
+// them next, so the build ends with a synchronisation.
+static gmg_status build_soa(gmg_wilson* h, bool f64, cudaStream_t s, bool* ok) {
+  DevBuf &g = f64 ? h->soa_gauge : h->soa_gauge_f, &c = f64 ? h->soa_clover : h->soa_clover_f;
+  bool& built = f64 ? h->soa_ok : h->soa_f_ok;
+  *ok = built;
+  if (built) return GMG_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  GMG_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return GMG_OK;
+  const int64_t V = h->dims.vol(), n = (V + kSoa - 1) / kSoa * kSoa * 36;
+  const size_t bytes = (size_t)n * (f64 ? sizeof(double2) : sizeof(float2));
+  if (g.alloc(bytes) != GMG_OK || c.alloc(bytes) != GMG_OK) {
+    cudaGetLastError();
+    g.free();
+    return GMG_OK;
   }
+  const int grid = (int)std::min<int64_t>((n + 255) / 256, 148 * 64);
+  if (f64)
+    soa_kernel<double2><<<grid, 256, 0, s>>>(h->gauge.as<double2>(), h->clover.as<double2>(), g.as<double2>(),
+                                             c.as<double2>(), V);
+  else
+    soa_kernel<float2><<<grid, 256, 0, s>>>(h->gauge_f.as<float2>(), h->clover_f.as<float2>(), g.as<float2>(),
+                                            c.as<float2>(), V);
   GMG_CUDA(cudaGetLastError());
+  GMG_CUDA(cudaStreamSynchronize(s));
+  *ok = built = true;
   return GMG_OK;
+}
+
+static gmg_status launch_site(gmg_wilson* h, int op, int dir, int disp, int vec_prec, int nrhs, const void* in,
+                              void* out, cudaStream_t s, bool* launched) {
+  const int64_t V = h->dims.vol(), grid = (V + kSoaThreads - 1) / kSoaThreads * nrhs;
+  *launched = false;
+  if (grid >= ((int64_t)1 << 31)) return GMG_OK;
+  GMG_TRY(build_soa(h, vec_prec == GMG_F64, s, launched));
+  if (!*launched) return GMG_OK;
+  const int tvol = h->dims.d[0] * h->dims.d[1] * h->dims.d[2];
+  const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
+  auto go = [&](auto kern, auto diag, const DevBuf& g, const DevBuf& c) -> gmg_status {
+    typedef typename wt<decltype(diag)>::C C;
+    kern<<<(unsigned)grid, kSoaThreads, 0, s>>>(g.as<C>(), c.as<C>(), h->nbr.as<int32_t>(), (const C*)in, (C*)out,
+                                                (int)V, nrhs, diag, op, dir, disp, h->apbc, tvol, h->dims.d[3]);
+    GMG_CUDA(cudaGetLastError());
+    return GMG_OK;
+  };
+  if (vec_prec == GMG_F64) {
+    const double diag = 4.0 + h->mass;
+    if (al & 31) return go(wilson_kernel<double, 0>, diag, h->soa_gauge, h->soa_clover);
+    return go(wilson_kernel<double, 2>, diag, h->soa_gauge, h->soa_clover);
+  }
+  const float diag = (float)(4.0 + h->mass);
+  if (al & 15) return go(wilson_kernel<float, 0>, diag, h->soa_gauge_f, h->soa_clover_f);
+  if (al & 31) return go(wilson_kernel<float, 1>, diag, h->soa_gauge_f, h->soa_clover_f);
+  return go(wilson_kernel<float, 2>, diag, h->soa_gauge_f, h->soa_clover_f);
 }
 
 // Grid of the tile kernels: one resident wave (the CTAs loop over the tiles),
@@ -1604,7 +1729,7 @@ static gmg_status run_variant(gmg_wilson* h, int v, bool dots, int op, int dir, 
   switch (v) {
     case GMG_WILSON_SITE:
       if (dots) break;
-      return launch_site(h, op, dir, disp, vec_prec, nrhs, in, out, s);
+      return launch_site(h, op, dir, disp, vec_prec, nrhs, in, out, s, launched);
     case GMG_WILSON_TILE:
       if (((uintptr_t)in | (uintptr_t)out) & 15) break;  // 16-byte spinor accesses
       return dots ? launch_tile<true>(h, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s)
@@ -1662,14 +1787,17 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     if (launched) return GMG_OK;
   }
   std::vector<int> cand;
-  if (!dots && nrhs < 4) cand.push_back(GMG_WILSON_SITE);
+  if (!dots && nrhs < 8) cand.push_back(GMG_WILSON_SITE);
   cand.push_back(GMG_WILSON_TILE);
   if (vec_prec == GMG_F32) {
     cand.push_back(kTileOcc3);
     cand.push_back(kTileOcc3Pf);
   }
-  cand.push_back(GMG_WILSON_QUAD);
-  if (nrhs >= 4) cand.push_back(GMG_WILSON_STAGED);
+  // the quad and staged kernels run when forced, the quad kernel also where the
+  // others do not apply (fields below 16-byte alignment); timing them on first calls
+  // found no key they win (8^4 to 32^4, 1 to 24 right-hand sides, both precisions)
+  // and took up to two thirds of such a call
+  if (((uintptr_t)in | (uintptr_t)out) & 15) cand.push_back(GMG_WILSON_QUAD);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GMG_CUDA(cudaStreamIsCapturing(s, &cap));
   int best = nrhs >= 4 ? GMG_WILSON_TILE : (dots ? GMG_WILSON_QUAD : GMG_WILSON_SITE);
@@ -1703,6 +1831,9 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   }
   GMG_TRY(zero_dots());
   GMG_TRY(run_variant(h, best, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));
+  // the site kernel without its copies (a stream being captured): the quad kernel takes every call
+  if (!launched && best == GMG_WILSON_SITE)
+    GMG_TRY(run_variant(h, GMG_WILSON_QUAD, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));
   if (!launched) return fail(GMG_ERR_UNSUPPORTED, "wilson apply: no kernel variant applies");
   return GMG_OK;
 }
