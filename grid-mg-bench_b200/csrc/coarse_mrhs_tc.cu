@@ -930,6 +930,12 @@ static gmg_status launch_stencil(gmg_coarse* h, const uint4* packed, int V, cons
   Shape sh;
   bool have = h->tc_force && make_shape(h->tc_force >> 8, h->tc_force & 0xff, npts, per_point, ncols, &sh);
   auto it = h->tc_shape.find(key);
+  // the choice of an earlier handle of the same sizes
+  const TuneKey shared = {0, dev, (int64_t)key, h->dims.d[0], h->dims.d[1], h->dims.d[2], h->dims.d[3]};
+  if (!have && it == h->tc_shape.end()) {
+    uint32_t c = 0;
+    if (tuned_find(shared, &c)) it = h->tc_shape.emplace(key, c).first;
+  }
   if (!have)
     have = it != h->tc_shape.end() && make_shape(it->second >> 8, it->second & 0xff, npts, per_point, ncols, &sh);
   if (!have) {
@@ -1003,6 +1009,7 @@ static gmg_status launch_stencil(gmg_coarse* h, const uint4* packed, int V, cons
       GMG_TRY(st);
       if (timing_ok) {
         h->tc_shape[key] = ((uint32_t)sh.ctas << 8) | (uint32_t)sh.pps;
+        tuned_store(shared, h->tc_shape[key]);
       } else {
         (void)cudaGetLastError();  // reset the error state the failed event call left behind
         sh = cand[0];

@@ -1,6 +1,8 @@
 // common.cu -- error state, device buffers, lattice tables.
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "gmg_internal.cuh"
@@ -54,6 +56,32 @@ void DevBuf::free() {
   if (p) cudaFree(p);
   p = nullptr;
   bytes = 0;
+}
+
+// ---------------------------------------------------------------------------
+// Launch choices found by timing, shared by the handles of a process: they
+// depend on the device and the sizes alone, so a second handle of the same
+// sizes does not time again.  Bounded; safe with several threads.
+// ---------------------------------------------------------------------------
+static std::mutex g_tuned_mu;
+static std::map<TuneKey, uint32_t>& tuned_map() {
+  static std::map<TuneKey, uint32_t> m;
+  return m;
+}
+constexpr size_t kMaxTuned = 4096;
+
+bool tuned_find(const TuneKey& key, uint32_t* choice) {
+  std::lock_guard<std::mutex> g(g_tuned_mu);
+  const auto it = tuned_map().find(key);
+  if (it == tuned_map().end()) return false;
+  *choice = it->second;
+  return true;
+}
+
+void tuned_store(const TuneKey& key, uint32_t choice) {
+  std::lock_guard<std::mutex> g(g_tuned_mu);
+  if (tuned_map().size() >= kMaxTuned) tuned_map().clear();
+  tuned_map()[key] = choice;
 }
 
 // nbr[p][s]: p<4 -> x + e_p, 4<=p<8 -> x - e_{p-4}, 8 -> x  (periodic wrap)

@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <array>
 #include <map>
 #include <string>
 #include <vector>
@@ -165,6 +166,12 @@ struct gmg_wilson {
 };
 
 namespace gmg {
+
+// launch choices found by timing, kept for the process (common.cu): what is
+// tuned, the device, and the sizes it depends on
+typedef std::array<int64_t, 7> TuneKey;
+bool tuned_find(const TuneKey& key, uint32_t* choice);
+void tuned_store(const TuneKey& key, uint32_t choice);
 
 // neighbour table (device) for a lattice
 gmg_status build_neighbors(const Dims& d, DevBuf& nbr, cudaStream_t s);

@@ -1781,6 +1781,18 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   const uint64_t key = (uint64_t)vec_prec | ((uint64_t)dots << 4) | ((uint64_t)(op == GMG_OP_MDIR) << 5) |
                        ((uint64_t)cls << 8);
   auto it = h->wtune.find(key);
+  // the choice of an earlier handle on the same lattice (fields of lesser
+  // alignment, which some variants refuse, are timed on their own)
+  TuneKey shared = {};
+  if (it == h->wtune.end()) {
+    int dev = 0;
+    GMG_CUDA(cudaGetDevice(&dev));
+    const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
+    shared = {1, dev, (int64_t)(key << 2 | (al & 15 ? 2 : al & 31 ? 1 : 0)), h->dims.d[0], h->dims.d[1], h->dims.d[2],
+              h->dims.d[3]};
+    uint32_t c = 0;
+    if (tuned_find(shared, &c)) it = h->wtune.emplace(key, (int)c).first;
+  }
   if (it != h->wtune.end()) {
     GMG_TRY(zero_dots());
     GMG_TRY(run_variant(h, it->second, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));
@@ -1828,6 +1840,7 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     GMG_TRY(st);
     GMG_CUDA(cudaGetLastError());
     h->wtune[key] = best;
+    if (shared[0]) tuned_store(shared, (uint32_t)best);
   }
   GMG_TRY(zero_dots());
   GMG_TRY(run_variant(h, best, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));

@@ -100,8 +100,9 @@ gmg_status gmg_coarse_apply(gmg_coarse* h, gmg_op op, int point, gmg_prec comput
    handle: CTAs per SM and stencil points per stage, for an apply of nrhs
    right-hand sides over npoints stencil points (9 for M) in `compute`
    (GMG_BF16 / GMG_F16); 0, 0 before the first such apply.  The first apply
-   of each (nbasis, padded nrhs, volume, point count, operand kind) times every
-   shape that fits and keeps the fastest, each timed launch after a write of a
+   of each (nbasis, padded nrhs, lattice, point count, operand kind) in a process
+   times every shape that fits and keeps the fastest (for later handles of the same
+   sizes too), each timed launch after a write of a
    192 MB buffer that evicts L2 (as a solve's other work does); that buffer is
    allocated on the first tuning call on a device and kept for the process.
    No counterpart in the reference. */
@@ -288,7 +289,8 @@ gmg_status gmg_wilson_apply_f32_in(gmg_wilson* h, gmg_op op, int nrhs, const flo
 /* Kernel variants of the multi-RHS Wilson-clover apply.  By default the
    variant is autotuned: every applicable one is timed once per (vector
    precision, fused MR products or not, single-hop op or not, nrhs class) on
-   the first call that meets the key, and the fastest is kept in the handle.
+   the first call in the process that meets the key on a lattice, and the fastest
+   is kept in the handle and for later handles of the same lattice.
    gmg_wilson_set_kernel forces one (GMG_WILSON_AUTO restores tuning); a forced
    variant that does not apply to a call falls back to the tuned choice. */
 typedef enum {
