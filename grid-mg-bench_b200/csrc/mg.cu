@@ -348,6 +348,10 @@ gmg_status mr_smooth(gmg_mg* h, int l, const Vec& b, Vec& x, int iters, cudaStre
       GMG_TRY(vec_mr_update(d1, d2, x, r, Ar, s, it + 1 < iters));
     } else {
       GMG_TRY(apply_op(h, l, r, Ar, s));
+      if (rhs_fused(x, 1)) {
+        GMG_TRY(rhs_mr_step(x, r, Ar, it + 1 < iters, s));
+        continue;
+      }
       // one sweep for both products: d1 = <r, Ar> (the conjugate of <Ar, r>), d2 = <Ar, Ar>
       GMG_TRY(vec_multidot(r, 2, r.elems(), Ar, d1, nullptr, s));
       GMG_TRY(vec_mr_update(d1, d2, x, r, Ar, s, it + 1 < iters, true));
@@ -567,11 +571,15 @@ gmg_status fgmres(gmg_mg* h, int l, const Vec& b, Vec& x, const Krylov& K, int m
       double2* dw = dh2 + nc;
       // pass 1: dh = V^H w; then w -= V dh fused with pass 2's dh2 = V^H w;
       // then w -= V dh2 fused with dw = |w|^2
-      GMG_TRY(vec_multidot(V0, j + 1, vstride, w, dh, nullptr, s));
-      GMG_TRY(vec_multiaxpy_dot(dh, V0, j + 1, vstride, w, s, -1.0, dh2, 1));
-      GMG_TRY(vec_multiaxpy_dot(dh2, V0, j + 1, vstride, w, s, -1.0, dw, 2));
       Vec vn = nth(V0, j + 1);
-      GMG_TRY(vec_scale_inv_norm(dw, w, vn, s));
+      if (l > 0 && V0.prec == w.prec && rhs_fused(w, m)) {
+        GMG_TRY(rhs_gs_step(V0, vstride, j + 1, w, vn, dh, dh2, dw, RhsGivens{}, s));
+      } else {
+        GMG_TRY(vec_multidot(V0, j + 1, vstride, w, dh, nullptr, s));
+        GMG_TRY(vec_multiaxpy_dot(dh, V0, j + 1, vstride, w, s, -1.0, dh2, 1));
+        GMG_TRY(vec_multiaxpy_dot(dh2, V0, j + 1, vstride, w, s, -1.0, dw, 2));
+        GMG_TRY(vec_scale_inv_norm(dw, w, vn, s));
+      }
       std::vector<zc> col;
       GMG_TRY(download(h, dh, (int)(2 * nc + R), col, s));
       std::vector<zc> hc(nc);
@@ -874,8 +882,13 @@ gmg_status fgmres_cap(gmg_mg* h, int l, const Vec& b, Vec& x, const Krylov& K, i
   double2* Y = L.gY.as<double2>();
   double* RES = L.gRes.as<double>();
   const int threads = (R + 31) / 32 * 32;
-  GMG_TRY(vec_multidot(b, 1, 0, b, bn2, nullptr, s));
-  GMG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), s));
+  // every step's vector work in one kernel per step where the level's vectors allow
+  const bool fused = V0.prec == w.prec && b.prec == w.prec && x.prec == w.prec && rhs_fused(w, m) && rhs_fused(b, m);
+  RhsGivens gv{H, G, CS, SN, RES, bn2, ctr, tol, m, maxit, 0, 0};
+  if (!fused) {
+    GMG_TRY(vec_multidot(b, 1, 0, b, bn2, nullptr, s));
+    GMG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), s));
+  }
   const int ncyc = std::max(1, (maxit + m - 1) / m);
   std::vector<cudaGraphConditionalHandle> hcyc(ncyc, 0);
   for (int c = 1; c < ncyc; ++c) GMG_TRY(cap_handle(s, &hcyc[c]));
@@ -890,13 +903,18 @@ gmg_status fgmres_cap(gmg_mg* h, int l, const Vec& b, Vec& x, const Krylov& K, i
     // r0 = b - A x, |r0|, v_0
     Vec v0 = nth(V0, 0);
     GMG_TRY(apply_op(h, l, x, w, sc));
-    GMG_TRY(vec_xmy(b, w, sc));
-    GMG_TRY(vec_multidot(w, 1, 0, w, beta2, nullptr, sc));
     std::vector<cudaGraphConditionalHandle> hit(m, 0);
     for (int j = 0; j < m; ++j) GMG_TRY(cap_handle(sc, &hit[j]));
-    cycle_init_kernel<<<1, threads, 0, sc>>>(beta2, bn2, R, m, G, RES, tol, ctr, maxit, hit[0]);
-    GMG_CUDA(cudaGetLastError());
-    GMG_TRY(vec_scale_inv_norm(beta2, w, v0, sc));
+    gv.next = hit[0];
+    if (fused) {
+      GMG_TRY(rhs_cycle_start(b, w, v0, c == 0, bn2, gv, sc));
+    } else {
+      GMG_TRY(vec_xmy(b, w, sc));
+      GMG_TRY(vec_multidot(w, 1, 0, w, beta2, nullptr, sc));
+      cycle_init_kernel<<<1, threads, 0, sc>>>(beta2, bn2, R, m, G, RES, tol, ctr, maxit, hit[0]);
+      GMG_CUDA(cudaGetLastError());
+      GMG_TRY(vec_scale_inv_norm(beta2, w, v0, sc));
+    }
     for (int j = 0; j < m; ++j) {
       cudaStream_t si = h->cap_st[dc + 1];
       GMG_TRY(cap_if_begin(sc, hit[j], si));
@@ -913,20 +931,32 @@ gmg_status fgmres_cap(gmg_mg* h, int l, const Vec& b, Vec& x, const Krylov& K, i
       double2* dh = h->dscr.as<double2>();
       double2* dh2 = dh + nc;
       double2* dw = dh2 + nc;
+      Vec vn = nth(V0, j + 1);
+      if (fused) {
+        gv.has_next = j + 1 < m;
+        gv.next = j + 1 < m ? hit[j + 1] : hit[j];
+        GMG_TRY(rhs_gs_step(V0, vstride, j + 1, w, vn, dh, dh2, dw, gv, si));
+        GMG_TRY(cap_if_end(si));
+        continue;
+      }
       GMG_TRY(vec_multidot(V0, j + 1, vstride, w, dh, nullptr, si));
       GMG_TRY(vec_multiaxpy_dot(dh, V0, j + 1, vstride, w, si, -1.0, dh2, 1));
       GMG_TRY(vec_multiaxpy_dot(dh2, V0, j + 1, vstride, w, si, -1.0, dw, 2));
-      Vec vn = nth(V0, j + 1);
       GMG_TRY(vec_scale_inv_norm(dw, w, vn, si));
       arnoldi_step_kernel<<<1, threads, 0, si>>>(dh, dh2, dw, j, m, R, H, G, CS, SN, RES, bn2, tol, ctr, maxit,
                                                  j + 1 < m ? hit[j + 1] : hit[j], j + 1 < m ? 1 : 0);
       GMG_CUDA(cudaGetLastError());
       GMG_TRY(cap_if_end(si));
     }
-    cycle_finish_kernel<<<1, threads, 0, sc>>>(H, G, R, m, ctr, maxit, Y, c + 1 < ncyc ? hcyc[c + 1] : hit[0],
-                                               c + 1 < ncyc ? 1 : 0);
-    GMG_CUDA(cudaGetLastError());
-    GMG_TRY(vec_multiaxpy(Y, flexible ? Z0 : V0, m, flexible ? zstride : vstride, x, sc, 1.0));
+    gv.has_next = c + 1 < ncyc;
+    gv.next = c + 1 < ncyc ? hcyc[c + 1] : hit[0];
+    if (fused && (!flexible || Z0.prec == x.prec)) {
+      GMG_TRY(rhs_cycle_finish(flexible ? Z0 : V0, flexible ? zstride : vstride, x, gv, sc));
+    } else {
+      cycle_finish_kernel<<<1, threads, 0, sc>>>(H, G, R, m, ctr, maxit, Y, gv.next, gv.has_next);
+      GMG_CUDA(cudaGetLastError());
+      GMG_TRY(vec_multiaxpy(Y, flexible ? Z0 : V0, m, flexible ? zstride : vstride, x, sc, 1.0));
+    }
     if (c > 0) GMG_TRY(cap_if_end(sc));
   }
   return GMG_OK;
@@ -978,6 +1008,7 @@ gmg_status graph_state(gmg_mg* h) {
     GMG_TRY(L.gRes.alloc(sizeof(double) * (size_t)R));
     GMG_TRY(L.gY.alloc(sizeof(double2) * (size_t)R * m));
     GMG_TRY(L.gCtr.alloc(sizeof(int) * 4));
+    GMG_CUDA(cudaMemset(L.gCtr.p, 0, sizeof(int) * 4));
     GMG_TRY(L.gBn.alloc(sizeof(double2) * (size_t)R));
     GMG_TRY(L.gBeta.alloc(sizeof(double2) * (size_t)R));
     // the captured cycle combines all m Krylov / flexible directions with

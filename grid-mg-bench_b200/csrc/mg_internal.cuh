@@ -106,4 +106,33 @@ gmg_status bicg_scalar(int which, const double2* a, const double2* b, double2* s
 gmg_status bicg_vec(int which, Vec& a, const Vec& b, const Vec& c, const Vec& d, const Vec& e, const double2* sc,
                     cudaStream_t s);
 
+// One coarse-level solver step of every right-hand side in one kernel (mg_fused.cu).
+// State of a captured (F)GMRES: Hessenberg matrices, rotated residuals g, rotations,
+// residual estimates (per right-hand side), |b|^2, counters (iterations, steps of the
+// cycle, a scratch word at zero), and the conditional node the kernel switches.
+struct RhsGivens {
+  double2 *H, *g, *cs, *sn;
+  double* res;
+  const double2* bn2;
+  int* ctr;
+  double tol;
+  int m, maxit, has_next;
+  cudaGraphConditionalHandle next;
+};
+// whether the kernels take a field like v and Krylov bases of m vectors
+bool rhs_fused(const Vec& v, int m);
+// h1 = V^H w, w' = w - V h1, h2 = V^H w', w'' = w' - V h2, vn = w'' / |w''| over the
+// first nx vectors of V: h1, h2 ([nx][R]) and |w''|^2 ([R]) to dh, dh2, dw; w is not
+// written.  With gv.H, column nx - 1 of the captured solve's state and its next step.
+gmg_status rhs_gs_step(const Vec& V0, int64_t vstride, int nx, const Vec& w, Vec& vn, double2* dh, double2* dh2,
+                       double2* dw, const RhsGivens& gv, cudaStream_t s);
+// x += a r and, with update_r, r -= a Ar, a = <Ar, r> / <Ar, Ar> per right-hand side
+gmg_status rhs_mr_step(Vec& x, Vec& r, const Vec& Ar, bool update_r, cudaStream_t s);
+// v0 = (b - w) / |b - w| and the start of a captured cycle; form_bn: the solve's first,
+// bn2 = |b|^2 and the counters from zero
+gmg_status rhs_cycle_start(const Vec& b, const Vec& w, Vec& v0, bool form_bn, double2* bn2, const RhsGivens& gv,
+                           cudaStream_t s);
+// x += sum_j y_j z_j over the steps taken, y = H^-1 g; switches the next cycle
+gmg_status rhs_cycle_finish(const Vec& Z0, int64_t zstride, Vec& x, const RhsGivens& gv, cudaStream_t s);
+
 }  // namespace gmg
