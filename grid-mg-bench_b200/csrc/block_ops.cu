@@ -151,7 +151,10 @@ template <class Cx> struct ProjArgs {
   int nsel;
   // fine[site * fsite + r * frhs + k * fk].  face >= 0: a face field of the
   // Wilson operator's hop `face` instead, sites c * nsel + s, with the upper two
-  // spins only; the lower two are (row of gamma, see face_spin) upper ones
+  // spins only; the lower two are phases times upper ones (see face_spin), so
+  // that the sum runs over the upper components and conj(v_upper) + phase
+  // conj(v_lower): half the MMAs, two sites of 6 components a turn.  32^4, 4^4
+  // blocks, nbasis 40, one face of 40 vectors: 1.56 -> 1.34 ms.
   int64_t fsite;
   int frhs, fk, face;
   int units, rchunks, G, KS;
@@ -159,13 +162,13 @@ template <class Cx> struct ProjArgs {
 
 constexpr int kProjWarps = 8;
 
-// Lower spin s (2 or 3) of (1 -+ gamma_mu) psi is a phase (code 0: 1, 1: i, 2:
-// -1, 3: -i) times upper spin *from, for hop p (p < 4: +mu, the projector 1 -
+// The lower spin *low of (1 -+ gamma_mu) psi that is a phase (code 0: 1, 1: i, 2:
+// -1, 3: -i) times upper spin s, for hop p (p < 4: +mu, the projector 1 -
 // gamma_mu; p >= 4: -mu, 1 + gamma_mu), in the gamma basis of the fine operator.
-__device__ __forceinline__ int face_spin(int p, int s, int* from) {
+__device__ __forceinline__ int face_spin(int p, int s, int* low) {
   const int mu = p & 3;
-  *from = mu < 2 ? 3 - s : s - 2;
-  const int g = mu == 0 ? 3 : mu == 1 ? (s == 3 ? 2 : 0) : mu == 2 ? (s == 3 ? 1 : 3) : 0;
+  *low = mu < 2 ? 3 - s : s + 2;
+  const int g = mu == 0 ? 3 : mu == 1 ? (*low == 3 ? 2 : 0) : mu == 2 ? (*low == 3 ? 1 : 3) : 0;
   return (g + (p < 4 ? 2 : 0)) & 3;
 }
 
@@ -178,7 +181,7 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
   const int mc = u / a.rchunks, rc = u - mc * a.rchunks;
   const int kk = lane & 3, part = (lane >> 2) & 1;
   const int64_t c = blockIdx.x, K = (int64_t)a.bv * dof;
-  const int nsites = a.sel ? a.nsel : a.bv;
+  const int nsites = FACE ? (a.nsel + 1) / 2 : a.sel ? a.nsel : a.bv;  // pairs of sites of a face
   double acc[MT][RQ][2];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -197,68 +200,93 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
 #pragma unroll
     for (int q = 0; q < RQ; ++q) foff[q] = min((rc * RQ + q) * 4 + (lane >> 3), a.nrhs - 1) * a.frhs;
     const uint32_t s1 = f64mma::second_sign(part, true);
-    int from2 = 0, from3 = 0, code2 = 0, code3 = 0;
+    int low0 = 0, low1 = 0, code0 = 0, code1 = 0;
     if (FACE) {
-      code2 = face_spin(a.face, 2, &from2);
-      code3 = face_spin(a.face, 3, &from3);
+      code0 = face_spin(a.face, 0, &low0);
+      code1 = face_spin(a.face, 1, &low1);
     }
-    Cx av[2][MT], fv[2][RQ];
+    constexpr int AT = FACE ? 2 * MT : MT;  // FACE: the upper components, then the lower ones
+    Cx av[2][AT], fv[2][RQ];
     int s = ks, k4 = 0, kc = kk, left = (nsites - ks + a.KS - 1) / a.KS * ((dof + 3) / 4);
-    // the site requested next and the one after it
-    int sb = a.sel ? a.sel[s] : s, sf = FACE ? s : blk[sb];
-    int sb1 = 0, sf1 = 0;
+    // the site requested next and the one after it (FACE: the pair's second site is sc)
+    auto second = [&](int pair) { return 2 * pair + 1 < a.nsel ? a.sel[2 * pair + 1] : -1; };
+    int sb = FACE ? a.sel[2 * s] : a.sel ? a.sel[s] : s, sf = FACE ? s : blk[sb], sc = FACE ? second(s) : 0;
+    int sb1 = 0, sf1 = 0, sc1 = 0;
     const Cx *Vp, *Fp;
     auto at_site = [&]() {
       Vp = Vb + (int64_t)sb * dof;
-      Fp = a.fine + (FACE ? c * a.nsel + sf : (int64_t)sf) * a.fsite;
+      Fp = a.fine + (FACE ? c * a.nsel + 2 * sf : (int64_t)sf) * a.fsite;
       s += a.KS;
       if (s < nsites) {
-        sb1 = a.sel ? a.sel[s] : s;
+        sb1 = FACE ? a.sel[2 * s] : a.sel ? a.sel[s] : s;
         sf1 = FACE ? s : blk[sb1];
+        if (FACE) sc1 = second(s);
       }
     };
-    auto request = [&](Cx (&A)[MT], Cx (&F)[RQ]) {
-      const int k = k4 + kk;
-      const bool in_k = k < dof;
+    auto request = [&](Cx (&A)[AT], Cx (&F)[RQ]) {
+      int k = k4 + kk;
+      bool in_k = k < dof;
+      const Cx *V = Vp, *Ff = Fp;
+      if (FACE && k >= 6) {
+        k -= 6;
+        in_k = sc >= 0;
+        if (in_k) {
+          V = Vb + (int64_t)sc * dof;
+          Ff = Fp + a.fsite;
+        }
+      }
+      auto basis = [&](int m, int at) {
+        return in_k ? __ldg(reinterpret_cast<const Cx*>(reinterpret_cast<const char*>(V + at) + (uint64_t)row[m] * Kb))
+                    : Cx{0, 0};
+      };
 #pragma unroll
-      for (int m = 0; m < MT; ++m) A[m] = in_k ? __ldg(reinterpret_cast<const Cx*>(reinterpret_cast<const char*>(Vp + k) + (uint64_t)row[m] * Kb)) : Cx{0, 0};
+      for (int m = 0; m < MT; ++m) A[m] = basis(m, k);
+      if constexpr (FACE) {
+        const int kl = k < 3 ? 3 * low0 + k : 3 * low1 + k - 3;
 #pragma unroll
-      int kf = k;  // component stored for k
-      if (FACE && k >= 6) kf = k < 9 ? from2 * 3 + k - 6 : from3 * 3 + k - 9;
+        for (int m = 0; m < MT; ++m) A[MT + m] = basis(m, kl);
+      }
 #pragma unroll
-      for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(Fp + foff[q] + kf * a.fk) : Cx{0, 0};
+      for (int q = 0; q < RQ; ++q) F[q] = in_k ? __ldg(Ff + foff[q] + k * a.fk) : Cx{0, 0};
       k4 += 4;
       if (k4 >= dof) {
         k4 = 0;
         sb = sb1;
         sf = sf1;
+        sc = sc1;
         at_site();
       }
     };
-    auto multiply = [&](const Cx (&A)[MT], const Cx (&F)[RQ]) {
-      double b0[RQ], b1[RQ];
-      if (FACE) {
-        // the phase as an exchange of the parts and signs of its own: i (x + i y) = -y + i x
-        const int code = kc < 6 ? 0 : kc < 9 ? code2 : code3;
+    auto multiply = [&](const Cx (&A)[AT], const Cx (&F)[RQ]) {
+      double b0[RQ], b1[RQ], ax[MT], ay[MT];
+#pragma unroll
+      for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, 0u, s1, b0[q], b1[q]);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        ax[m] = (double)A[m].x;
+        ay[m] = (double)A[m].y;
+      }
+      if constexpr (FACE) {
+        // + conj(phase) v_lower, the phase as an exchange of the parts and signs: -i (x + i y) = y - i x
+        const int code = kc % 6 < 3 ? code0 : code1;
         const bool swap = code & 1;
-        const uint32_t neg = (code & 2) ? 0x80000000u : 0u;
-        const uint32_t nre = neg ^ (swap ? 0x80000000u : 0u);  // sign of the real part's source, of the imaginary's: neg
+        const uint32_t nre = code >= 2 ? 0x80000000u : 0u, nim = nre ^ (swap ? 0x80000000u : 0u);
 #pragma unroll
-        for (int q = 0; q < RQ; ++q)
-          f64mma::expand(F[q], part ^ (swap ? 1 : 0), part ? neg : nre, (part ? nre : neg) ^ s1, b0[q], b1[q]);
+        for (int m = 0; m < MT; ++m) {
+          const Cx l = A[MT + m];
+          ax[m] += f64mma::flip(swap ? l.y : l.x, nre);
+          ay[m] += f64mma::flip(swap ? l.x : l.y, nim);
+        }
         kc = kc + 4 >= dof ? kk : kc + 4;
-      } else {
-#pragma unroll
-        for (int q = 0; q < RQ; ++q) f64mma::expand(F[q], part, 0u, s1, b0[q], b1[q]);
       }
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].x, b0[q]);
+        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], ax[m], b0[q]);
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], (double)A[m].y, b1[q]);
+        for (int q = 0; q < RQ; ++q) f64mma::mma(acc[m][q], ay[m], b1[q]);
     };
     at_site();
     request(av[0], fv[0]);
@@ -331,17 +359,21 @@ static gmg_status launch_project(const ProjArgs<typename ctype<T>::t>& a, int Vc
 // 8), small tiles and part-filled chips in CTAs of 8 (16^4, nbasis 24, 12 RHS:
 // 95 us, 118 with 4).  16^4, nbasis 32, 32 RHS: 290 us with w = 2 and own CTAs,
 // 376 with w = 4 and shared ones; 8^4 with 16 blocks, nbasis 24, 24 RHS: 37 us
-// with w = 1, 98 with w = 3.
+// with w = 1, 98 with w = 3.  A face reads its basis twice as fast per MMA and
+// holds two loads a row: with blocks enough to fill the chip several times over,
+// the units of a block share a CTA, tiles of up to 3 quads (32^4, 40 columns:
+// 1.34 ms; 1.84 in CTAs of their own, 1.49 with w = 5).
 struct ProjShape {
   int w, chunks, G, KS;
 };
-static ProjShape project_shape(int Vc, int MT, int mchunks, int rq) {
+static ProjShape project_shape(int Vc, int MT, int mchunks, int rq, bool face) {
   ProjShape best{1, rq, 1, kProjWarps};
   double t_best = 1e30;
-  for (int w = 1; w <= std::min(5, rq); ++w) {
+  face = face && Vc >= 148 * 8;
+  for (int w = 1; w <= std::min(face ? 3 : 5, rq); ++w) {
     const int chunks = (rq + w - 1) / w, units = mchunks * chunks;
     const int regs = (40 + 4 * MT * w + 8 * MT + 8 * w + 7) / 8 * 8;
-    for (int shared = 0; shared < 2; ++shared) {
+    for (int shared = face ? 1 : 0; shared < 2; ++shared) {
       int warps = MT * w > 10 ? 4 : kProjWarps;
       int G = shared ? std::min(units, warps) : 1;
       int64_t ctas = (int64_t)Vc * ((units + G - 1) / G);
@@ -375,7 +407,7 @@ static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const voi
   GMG_CHECK((int64_t)h->bv * h->dof < ((int64_t)1 << 28), GMG_ERR_UNSUPPORTED, "project: more than 2^28 components per block");
   const int mt = (h->N + 7) / 8, mchunks = (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
   const int Vc = (int)h->cdims.vol();
-  const ProjShape sh = project_shape(Vc, MT, mchunks, (nrhs + 3) / 4);
+  const ProjShape sh = project_shape(Vc, MT, mchunks, (nrhs + 3) / 4, FACE);
   const ProjArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
                        reinterpret_cast<const Cx*>(fine), reinterpret_cast<Cx*>(out), cstr, rstr, istr, h->N, h->dof,
                        h->bv, nrhs, sel, nsel, (int64_t)nrhs * (FACE ? 6 : h->dof), cmajor ? 1 : h->dof,
