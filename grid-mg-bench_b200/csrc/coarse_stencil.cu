@@ -496,7 +496,6 @@ static bool launch_simt_pipe(const LinkSel& L, const void* in, void* out, int V,
   if (smem > 72 * 1024) return false;
   const int threads = std::max(32, ((N / TB) * (R / TR) + 31) / 32 * 32);
   auto kern = N == 32 ? coarse_simt_pipe_kernel<T, TR, TB, 32>
-             : N == 24 ? coarse_simt_pipe_kernel<T, TR, TB, 24>
              : N == 40 ? coarse_simt_pipe_kernel<T, TR, TB, 40>
                        : coarse_simt_pipe_kernel<T, TR, TB, 0>;
   *st = GMG_OK;
