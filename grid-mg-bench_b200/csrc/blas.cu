@@ -452,8 +452,18 @@ __device__ __forceinline__ void st_pair(double2* p, int64_t e, double ur, double
 // A thread takes two consecutive complex numbers of a site's R x dof row (dof
 // even, so both belong to one RHS): twice the bytes in flight per thread for
 // the same product accumulators, which bound the kernels' occupancy.
+// dots_min_ctas, update_min_ctas: given one CTA per SM as its target the compiler keeps the loads of an FP32
+// batch together where its own balance of registers and occupancy splits them (dots,
+// 16^4 x 24 RHS: NV 5 359 -> 186 us, NV 1 to 4 2 to 5 % faster, NV 6 206 -> 257; update:
+// NV 1, 3, 4 7 to 11 % faster, NV 2 and 5 10 % slower); 0 leaves it to the compiler.
+template <class T> __host__ __device__ constexpr int dots_min_ctas(int nv) {
+  return sizeof(T) == 4 && nv >= 1 && nv <= 5 ? 1 : 0;
+}
+template <class T> __host__ __device__ constexpr int update_min_ctas(int nv) {
+  return sizeof(T) == 4 && (nv == 1 || nv == 3 || nv == 4) ? 1 : 0;
+}
 template <int NV, class T = double>
-__global__ void __launch_bounds__(kDcgsThreads) dcgs_dots_row_kernel(const typename C2<T>::t* __restrict__ V0,
+__global__ void __launch_bounds__(kDcgsThreads, dots_min_ctas<T>(NV)) dcgs_dots_row_kernel(const typename C2<T>::t* __restrict__ V0,
                                                                      int64_t vstride,
                                                                      const typename C2<T>::t* __restrict__ B, int64_t V,
                                                                      int R, int dof, int spb,
@@ -545,7 +555,7 @@ __global__ void __launch_bounds__(kDcgsThreads) dcgs_dots_row_kernel(const typen
 // next one after one projection).  cf per RHS: c[NV], g[NV], (1/alpha, 0),
 // d, (1/beta, 0), at cf[k * R + r].  Two complex numbers per thread.
 template <int NV, class T = double>
-__global__ void __launch_bounds__(kDcgsThreads) dcgs_update_row_kernel(const double2* __restrict__ cfg,
+__global__ void __launch_bounds__(kDcgsThreads, update_min_ctas<T>(NV)) dcgs_update_row_kernel(const double2* __restrict__ cfg,
                                                                        typename C2<T>::t* __restrict__ V0,
                                                                        int64_t vstride,
                                                                        const typename C2<T>::t* __restrict__ B,
