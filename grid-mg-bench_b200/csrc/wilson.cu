@@ -497,6 +497,19 @@ __global__ void soa_kernel(const C* __restrict__ gauge, const C* __restrict__ cl
   }
 }
 
+static gmg_status fill_soa(gmg_wilson* h, bool f64, cudaStream_t s) {
+  const int64_t V = h->dims.vol(), n = (V + kSoa - 1) / kSoa * kSoa * 36;
+  const int grid = (int)std::min<int64_t>((n + 255) / 256, 148 * 64);
+  if (f64)
+    soa_kernel<double2><<<grid, 256, 0, s>>>(h->gauge.as<double2>(), h->clover.as<double2>(),
+                                             h->soa_gauge.as<double2>(), h->soa_clover.as<double2>(), V);
+  else
+    soa_kernel<float2><<<grid, 256, 0, s>>>(h->gauge_f.as<float2>(), h->clover_f.as<float2>(),
+                                            h->soa_gauge_f.as<float2>(), h->soa_clover_f.as<float2>(), V);
+  GMG_CUDA(cudaGetLastError());
+  return GMG_OK;
+}
+
 template <class T, int VEC>
 __global__ void __launch_bounds__(kSoaThreads, sizeof(T) == 8 ? 3 : 6) wilson_kernel(
     const typename wt<T>::C* __restrict__ gauge, const typename wt<T>::C* __restrict__ clover,
@@ -1378,6 +1391,9 @@ __global__ void d2f_wilson(const double2* __restrict__ a, float2* __restrict__ b
 
 gmg_status wilson_build_clover(gmg_wilson* h, cudaStream_t s) {
   const int V = (int)h->dims.vol();
+  // the site kernel's copies that exist are filled again below, in place: a
+  // captured graph may hold them, and no later call need build them
+  const bool soa = h->soa_ok, soa_f = h->soa_f_ok;
   h->soa_ok = h->soa_f_ok = false;
   GMG_TRY(h->clover.alloc(sizeof(double2) * 72 * (size_t)V));
   GMG_TRY(h->clover_f.alloc(sizeof(float2) * 72 * (size_t)V));
@@ -1397,6 +1413,10 @@ gmg_status wilson_build_clover(gmg_wilson* h, cudaStream_t s) {
   hop_links_kernel<double2><<<g, 256, 0, s>>>(h->gauge.as<double2>(), h->nbr.as<int32_t>(), h->hop.as<double2>(), V);
   hop_links_kernel<float2><<<g, 256, 0, s>>>(h->gauge_f.as<float2>(), h->nbr.as<int32_t>(), h->hop_f.as<float2>(), V);
   GMG_CUDA(cudaGetLastError());
+  if (soa) GMG_TRY(fill_soa(h, true, s));
+  if (soa_f) GMG_TRY(fill_soa(h, false, s));
+  h->soa_ok = soa;
+  h->soa_f_ok = soa_f;
   return GMG_OK;
 }
 
@@ -1589,11 +1609,11 @@ static gmg_status launch_quad(gmg_wilson* h, int op, int dir, int disp, int vec_
   return GMG_OK;
 }
 
-// thread per (site, RHS), links and clover from global memory
 // The site kernel's copies of the links and the clover in precision f64 / f32, built
 // on the first launch that finds none (not while the stream is being captured, nor
-// when the device memory does not suffice: *ok = false).  Other streams may use
-// them next, so the build ends with a synchronisation.
+// when the device memory does not suffice: *ok = false) and filled again by every
+// wilson_build_clover.  Other streams may use them next, so the build ends with a
+// synchronisation.
 static gmg_status build_soa(gmg_wilson* h, bool f64, cudaStream_t s, bool* ok) {
   DevBuf &g = f64 ? h->soa_gauge : h->soa_gauge_f, &c = f64 ? h->soa_clover : h->soa_clover_f;
   bool& built = f64 ? h->soa_ok : h->soa_f_ok;
@@ -1609,14 +1629,7 @@ static gmg_status build_soa(gmg_wilson* h, bool f64, cudaStream_t s, bool* ok) {
     g.free();
     return GMG_OK;
   }
-  const int grid = (int)std::min<int64_t>((n + 255) / 256, 148 * 64);
-  if (f64)
-    soa_kernel<double2><<<grid, 256, 0, s>>>(h->gauge.as<double2>(), h->clover.as<double2>(), g.as<double2>(),
-                                             c.as<double2>(), V);
-  else
-    soa_kernel<float2><<<grid, 256, 0, s>>>(h->gauge_f.as<float2>(), h->clover_f.as<float2>(), g.as<float2>(),
-                                            c.as<float2>(), V);
-  GMG_CUDA(cudaGetLastError());
+  GMG_TRY(fill_soa(h, f64, s));
   GMG_CUDA(cudaStreamSynchronize(s));
   *ok = built = true;
   return GMG_OK;
