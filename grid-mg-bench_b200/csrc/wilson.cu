@@ -1635,6 +1635,12 @@ static gmg_status build_soa(gmg_wilson* h, bool f64, cudaStream_t s, bool* ok) {
   return GMG_OK;
 }
 
+static void drop_soa(gmg_wilson* h, bool f64) {
+  (f64 ? h->soa_ok : h->soa_f_ok) = false;
+  (f64 ? h->soa_gauge : h->soa_gauge_f).free();
+  (f64 ? h->soa_clover : h->soa_clover_f).free();
+}
+
 static gmg_status launch_site(gmg_wilson* h, int op, int dir, int disp, int vec_prec, int nrhs, const void* in,
                               void* out, cudaStream_t s, bool* launched) {
   const int64_t V = h->dims.vol(), grid = (V + kSoaThreads - 1) / kSoaThreads * nrhs;
@@ -1827,6 +1833,7 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   GMG_CUDA(cudaStreamIsCapturing(s, &cap));
   int best = nrhs >= 4 ? GMG_WILSON_TILE : (dots ? GMG_WILSON_QUAD : GMG_WILSON_SITE);
   if (cap == cudaStreamCaptureStatusNone) {
+    const bool f64 = vec_prec == GMG_F64, had_soa = f64 ? h->soa_ok : h->soa_f_ok;
     cudaEvent_t e0, e1;
     GMG_CUDA(cudaEventCreate(&e0));
     GMG_CUDA(cudaEventCreate(&e1));
@@ -1852,6 +1859,7 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     cudaEventDestroy(e1);
     GMG_TRY(st);
     GMG_CUDA(cudaGetLastError());
+    if (best != GMG_WILSON_SITE && !had_soa) drop_soa(h, f64);  // copies made for the timing alone
     h->wtune[key] = best;
     if (shared[0]) tuned_store(shared, (uint32_t)best);
   }

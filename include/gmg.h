@@ -269,7 +269,14 @@ gmg_status gmg_wilson_destroy(gmg_wilson* h);
 gmg_status gmg_wilson_set_gauge(gmg_wilson* h, const double* U, int on_device, gmg_stream s);
 /* Clover blocks [V][2][6][6] complex128 to host or device memory. */
 gmg_status gmg_wilson_get_clover(gmg_wilson* h, double* clover, int on_device, gmg_stream s);
-/* op M / Mdag / Mdiag / Mdir(dir, disp); fields [V][nrhs][12] of vec_prec (F64/F32). */
+/* op M / Mdag / Mdiag / Mdir(dir, disp); fields [V][nrhs][12] of vec_prec (F64/F32).
+   The kernel for fewer than 8 right-hand sides (GMG_WILSON_SITE) reads copies of the
+   links and the clover of its own, 1152 bytes per site in FP64 and 576 in FP32 (1.2
+   and 0.6 GB at 32^4): the first call of a precision that uses or times it allocates
+   them and synchronises the stream.  They are kept while that kernel is in use (freed
+   again where only the timing needed them), refilled by gmg_wilson_set_gauge, and
+   freed with the handle; without memory for them, or when that first call is in a
+   stream capture, another kernel runs. */
 gmg_status gmg_wilson_apply(gmg_wilson* h, gmg_op op, int dir, int disp, gmg_prec vec_prec,
                             int nrhs, const void* in, void* out, gmg_stream s);
 /* op M / Mdag in FP64 arithmetic on an FP32 input field, FP64 output: the same

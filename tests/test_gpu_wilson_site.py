@@ -47,3 +47,24 @@ def test_captured_apply_follows_set_gauge(prec, nrhs):
     _handle(872).M(x, ref)
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_copies_of_a_lost_timing_are_freed(prec):
+    # the copies stay allocated only where the site kernel is what later calls run
+    def run(dims):
+        w, v = _handle(873, None, dims), dims[0] * dims[1] * dims[2] * dims[3]
+        x = _field(prec, 7, 874, v)
+        out = torch.zeros_like(x)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        w.M(x, out)
+        torch.cuda.synchronize()
+        return w, w.tuned_kernel(prec, 7), free - torch.cuda.mem_get_info()[0]
+
+    run((4, 4, 4, 4))  # loads the kernels
+    dims = (20, 24, 20, 24)
+    copies = 230400 * 72 * (16 if prec == "f64" else 8)
+    w, kernel, taken = run(dims)
+    print(kernel, taken, copies)
+    assert taken < copies / 4 if kernel != "site" else taken >= copies, (kernel, taken)
