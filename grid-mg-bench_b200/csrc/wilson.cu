@@ -1865,8 +1865,10 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   }
   GMG_TRY(zero_dots());
   GMG_TRY(run_variant(h, best, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));
-  // the site kernel without its copies (a stream being captured): the quad kernel takes every call
-  if (!launched && best == GMG_WILSON_SITE)
+  // a choice that does not apply (while the stream is being captured nothing is timed: the
+  // site kernel without its copies, the tile kernel on fields below 16-byte alignment):
+  // the quad kernel takes every call
+  if (!launched)
     GMG_TRY(run_variant(h, GMG_WILSON_QUAD, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &launched));
   if (!launched) return fail(GMG_ERR_UNSUPPORTED, "wilson apply: no kernel variant applies");
   return GMG_OK;

@@ -68,3 +68,48 @@ def test_copies_of_a_lost_timing_are_freed(prec):
     w, kernel, taken = run(dims)
     print(kernel, taken, copies)
     assert taken < copies / 4 if kernel != "site" else taken >= copies, (kernel, taken)
+
+
+def _offset(prec, nrhs, stream, entries):
+    """A field whose first entry lies `entries` complex numbers into an aligned buffer."""
+    x = _field(prec, nrhs, stream)
+    buf = torch.zeros(x.numel() + entries, dtype=x.dtype, device="cuda")
+    buf[entries:] = x.reshape(-1)
+    return buf[entries:].view(x.shape)
+
+
+# squared relative deviation: sums of about 100 terms, rounded in the field's precision
+TOL = {"f64": 1e-28, "f32": 1e-12}
+
+
+def _oracle(x, op, gauge_stream):
+    import oracle as orc
+    U = inputs.hot_gauge(DIMS, inputs.rng(stream=gauge_stream))
+    return orc.wilson_clover(DIMS, U, orc.clover_build(DIMS, U, 1.0), -0.1, 1, x.cpu().numpy().astype("complex128"), op)
+
+
+def _deviation(ref, got):
+    import oracle as orc
+    return orc.rel_dev_sq(ref, got.cpu().numpy().astype("complex128"))
+
+
+@pytest.mark.parametrize("prec,entries", [("f64", 0), ("f64", 1), ("f32", 0), ("f32", 1), ("f32", 2)])
+@pytest.mark.parametrize("nrhs", [1, 3, 7])
+@pytest.mark.parametrize("op", ["M", "Mdag", "Mdiag"])
+def test_field_alignments(prec, entries, nrhs, op):
+    import oracle as orc
+    x, out = _offset(prec, nrhs, 875, entries), _offset(prec, nrhs, 876, entries)
+    getattr(_handle(877), op)(x, out)
+    assert _deviation(_oracle(x, {"M": orc.OP_M, "Mdag": orc.OP_MDAG, "Mdiag": orc.OP_MDIAG}[op], 877), out) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec,entries,nrhs", [("f64", 0, 1), ("f32", 0, 2), ("f32", 1, 2), ("f32", 1, 5), ("f32", 1, 9)])
+def test_first_call_in_a_capture(prec, entries, nrhs):
+    # no copies, and nothing timed: whatever runs has to take these fields
+    import oracle as orc
+    x, out = _offset(prec, nrhs, 878, entries), _offset(prec, nrhs, 879, entries)
+    w = _handle(880, None)
+    g = _captured(w, x, out)
+    g.replay()
+    torch.cuda.synchronize()
+    assert _deviation(_oracle(x, orc.OP_M, 880), out) < TOL[prec]
