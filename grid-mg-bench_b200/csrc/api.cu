@@ -424,10 +424,9 @@ gmg_status gmg_wilson_set_kernel(gmg_wilson* h, gmg_wilson_kernel k) {
 gmg_status gmg_wilson_tuned_kernel(gmg_wilson* h, gmg_prec vec_prec, int nrhs, int fused_mr, int single_hop,
                                    gmg_wilson_kernel* k) {
   GMG_CHECK(h && k, GMG_ERR_ARGUMENT, "gmg_wilson_tuned_kernel: null argument");
-  const int cls = nrhs < 4 ? 0 : nrhs < 8 ? 1 : nrhs < 16 ? 2 : nrhs < 32 ? 3 : 4;
-  const uint64_t key = (uint64_t)vec_prec | ((uint64_t)(fused_mr != 0) << 4) | ((uint64_t)(single_hop != 0) << 5) |
-                       ((uint64_t)cls << 8);
-  auto it = h->wtune.find(key);
+  auto it = h->wtune.end();  // the best aligned fields' choice, if there is one
+  for (int al = 0; al < 3 && it == h->wtune.end(); ++al)
+    it = h->wtune.find(wilson_tune_key(vec_prec, fused_mr != 0, single_hop != 0, nrhs, al));
   // internal register-budget sub-variants (ids >= 16) of the tile kernel report as TILE
   *k = it == h->wtune.end() ? GMG_WILSON_AUTO
                             : (gmg_wilson_kernel)(it->second >= 16 ? (int)GMG_WILSON_TILE : it->second);

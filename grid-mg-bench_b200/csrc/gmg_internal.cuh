@@ -162,7 +162,7 @@ struct gmg_wilson {
   std::map<int, PipePlan> pplans;
   gmg::DevBuf dev_err;    // device error word of the staged kernel
   int wforce = -1;                  // forced kernel variant (gmg_wilson_kernel), -1: autotuned
-  std::map<uint64_t, int> wtune;    // autotuned variant per (precision, products, op class, nrhs class)
+  std::map<uint64_t, int> wtune;    // autotuned variant per wilson_tune_key
 };
 
 namespace gmg {
@@ -171,6 +171,13 @@ namespace gmg {
 // tuned, the device, and the sizes it depends on
 typedef std::array<int64_t, 7> TuneKey;
 bool tuned_find(const TuneKey& key, uint32_t* choice);
+// what a Wilson-clover variant is chosen by: vector precision, fused products or not,
+// single-hop op or not, nrhs class, alignment class of the fields (0: 32 bytes, 1: 16, 2: less)
+inline uint64_t wilson_tune_key(int vec_prec, bool dots, bool single_hop, int nrhs, int align) {
+  const int cls = nrhs < 4 ? 0 : nrhs < 8 ? 1 : nrhs < 16 ? 2 : nrhs < 32 ? 3 : 4;
+  return (uint64_t)vec_prec | ((uint64_t)dots << 4) | ((uint64_t)single_hop << 5) | ((uint64_t)align << 6) |
+         ((uint64_t)cls << 8);
+}
 void tuned_store(const TuneKey& key, uint32_t choice);
 
 // neighbour table (device) for a lattice

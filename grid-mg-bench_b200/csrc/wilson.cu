@@ -1796,19 +1796,16 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     if (launched) return GMG_OK;
     // a forced variant that does not apply falls through to the tuned choice
   }
-  const int cls = nrhs < 4 ? 0 : nrhs < 8 ? 1 : nrhs < 16 ? 2 : nrhs < 32 ? 3 : 4;
-  const uint64_t key = (uint64_t)vec_prec | ((uint64_t)dots << 4) | ((uint64_t)(op == GMG_OP_MDIR) << 5) |
-                       ((uint64_t)cls << 8);
+  // fields of lesser alignment, which some variants refuse, are timed on their own
+  const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
+  const uint64_t key = wilson_tune_key(vec_prec, dots, op == GMG_OP_MDIR, nrhs, al & 15 ? 2 : al & 31 ? 1 : 0);
   auto it = h->wtune.find(key);
-  // the choice of an earlier handle on the same lattice (fields of lesser
-  // alignment, which some variants refuse, are timed on their own)
+  // the choice of an earlier handle on the same lattice
   TuneKey shared = {};
   if (it == h->wtune.end()) {
     int dev = 0;
     GMG_CUDA(cudaGetDevice(&dev));
-    const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
-    shared = {1, dev, (int64_t)(key << 2 | (al & 15 ? 2 : al & 31 ? 1 : 0)), h->dims.d[0], h->dims.d[1], h->dims.d[2],
-              h->dims.d[3]};
+    shared = {1, dev, (int64_t)key, h->dims.d[0], h->dims.d[1], h->dims.d[2], h->dims.d[3]};
     uint32_t c = 0;
     if (tuned_find(shared, &c)) it = h->wtune.emplace(key, (int)c).first;
   }

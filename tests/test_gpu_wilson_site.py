@@ -113,3 +113,16 @@ def test_first_call_in_a_capture(prec, entries, nrhs):
     g.replay()
     torch.cuda.synchronize()
     assert _deviation(_oracle(x, orc.OP_M, 880), out) < TOL[prec]
+
+
+def test_choices_by_alignment():
+    # a choice made for fields of 8-byte alignment, where few kernels apply, is not the aligned fields' one
+    dims = (16, 16, 16, 8)
+    w = _handle(881, None, dims)
+    x = _field("f32", 12, 882, 32768)
+    buf = torch.zeros(2 * x.numel() + 1, dtype=x.dtype, device="cuda")
+    lo, hi = buf[1:x.numel() + 1].view(x.shape), buf[x.numel() + 1:].view(x.shape)
+    w.M(lo, hi)
+    assert w.tuned_kernel("f32", 12) == "quad"
+    w.M(x, torch.zeros_like(x))
+    assert w.tuned_kernel("f32", 12) == "tile"
