@@ -994,8 +994,10 @@ gmg_status kcycle_cap(gmg_mg* h, int l, const Vec& in, Vec& out, int d) {
   return mr_smooth(h, l, in, out, h->P.smoother_iters, s);
 }
 
-// device state of the coarse-level solvers for max_rhs RHS (allocated before any capture)
-gmg_status graph_state(gmg_mg* h) {
+// device state of the coarse-level solvers for max_rhs RHS (allocated before any capture),
+// cleared on the solve's stream: the legacy default stream, which other streams need not
+// wait for, could clear it in the middle of a captured cycle
+gmg_status graph_state(gmg_mg* h, cudaStream_t s) {
   const int R = h->Rmax;
   for (size_t l = 1; l < h->L.size(); ++l) {
     MGLevel& L = *h->L[l];
@@ -1008,13 +1010,13 @@ gmg_status graph_state(gmg_mg* h) {
     GMG_TRY(L.gRes.alloc(sizeof(double) * (size_t)R));
     GMG_TRY(L.gY.alloc(sizeof(double2) * (size_t)R * m));
     GMG_TRY(L.gCtr.alloc(sizeof(int) * 4));
-    GMG_CUDA(cudaMemset(L.gCtr.p, 0, sizeof(int) * 4));
+    GMG_CUDA(cudaMemsetAsync(L.gCtr.p, 0, sizeof(int) * 4, s));
     GMG_TRY(L.gBn.alloc(sizeof(double2) * (size_t)R));
     GMG_TRY(L.gBeta.alloc(sizeof(double2) * (size_t)R));
     // the captured cycle combines all m Krylov / flexible directions with
     // zero coefficients beyond the steps taken: keep them finite
-    GMG_CUDA(cudaMemset(L.V0.p, 0, L.V0.buf.bytes));
-    if (L.Z0.p) GMG_CUDA(cudaMemset(L.Z0.p, 0, L.Z0.buf.bytes));
+    GMG_CUDA(cudaMemsetAsync(L.V0.p, 0, L.V0.buf.bytes, s));
+    if (L.Z0.p) GMG_CUDA(cudaMemsetAsync(L.Z0.p, 0, L.Z0.buf.bytes, s));
   }
   for (auto& st : h->cap_st)
     if (!st) GMG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -1026,9 +1028,9 @@ gmg_status graph_state(gmg_mg* h) {
 // solution buffers.  The fine-level steps (restriction, prolongation, MR
 // smoothing: a few large kernels) stay plain launches on the caller's vectors,
 // so the Krylov vectors need no copies in and out of fixed buffers.
-gmg_status build_kcycle_graph(gmg_mg* h, int R, cudaGraphExec_t* exec) {
+gmg_status build_kcycle_graph(gmg_mg* h, int R, cudaGraphExec_t* exec, cudaStream_t s) {
   *exec = nullptr;
-  GMG_TRY(graph_state(h));
+  GMG_TRY(graph_state(h, s));
   cudaStream_t s0 = h->cap_st[0];
   MGLevel& C = *h->L[1];
   Vec bc = C.bc.with_rhs(R), xc = C.xc.with_rhs(R);
@@ -1518,7 +1520,7 @@ extern "C" gmg_status gmg_mg_solve(gmg_mg* h, int nrhs, const double* b, double*
         GMG_TRY(kcycle(h, 0, src, out, s));
         GMG_CUDA(cudaStreamSynchronize(s));
         cudaGraphExec_t ex = nullptr;
-        if (build_kcycle_graph(h, Rb, &ex) == GMG_OK)
+        if (build_kcycle_graph(h, Rb, &ex, s) == GMG_OK)
           h->kgraph[Rb] = ex;
         else
           h->graph_broken = true;  // keep the host-driven cycle
