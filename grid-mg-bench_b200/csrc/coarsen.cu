@@ -215,6 +215,21 @@ static gmg_status coarsen_faces(gmg_coarse* out, gmg_agg* agg, const FineOpRef& 
   const int64_t Vc = out->dims.vol();
   GMG_TRY(out->links_ref.alloc(sizeof(double2) * 9 * Vc * N * N));  // every entry is written below
   GMG_TRY(coarsen_workspace(agg, s));
+  // the constructions of one aggregation share its workspace: one on another stream
+  // waits for the one before it (its event cannot enter a stream capture)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  GMG_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (cap == cudaStreamCaptureStatusNone) {
+    if (!agg->cw_done) GMG_CUDA(cudaEventCreateWithFlags(&agg->cw_done, cudaEventDisableTiming));
+    GMG_CUDA(cudaStreamWaitEvent(s, agg->cw_done, 0));
+  }
+  struct Done {
+    cudaEvent_t ev;
+    cudaStream_t s;
+    ~Done() {
+      if (ev) cudaEventRecord(ev, s);
+    }
+  } done{cap == cudaStreamCaptureStatusNone ? agg->cw_done : nullptr, s};
   const int nb = agg->cw_nb;
   double* phi = agg->cw_phi.as<double>();
   double* wf = agg->cw_w.as<double>();

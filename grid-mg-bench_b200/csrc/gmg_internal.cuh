@@ -135,6 +135,10 @@ struct gmg_agg {
   int cw_nb = 0;
   int cw_max_batch = 0;  // cap on basis vectors per CoarsenOperator batch (0: from free memory)
   int cw_nface[4] = {0, 0, 0, 0}, cw_nsel[4] = {0, 0, 0, 0};
+  cudaEvent_t cw_done = nullptr;  // the last construction's use of the workspace has ended
+  ~gmg_agg() {
+    if (cw_done) cudaEventDestroy(cw_done);
+  }
 };
 
 struct gmg_wilson {
