@@ -285,7 +285,9 @@ gmg_status gmg_agg_set_coarsen_batch(gmg_agg* h, int max_batch) {
   if (max_batch != h->cw_max_batch) {
     GMG_CUDA(cudaDeviceSynchronize());  // the kept workspace may still be in use
     h->cw_max_batch = max_batch;
-    h->cw_nb = 0;  // the workspace is rebuilt for the new batch on the next construction
+    h->cw_phi.free();  // rebuilt for the new batch on the next construction
+    h->cw_w.free();
+    h->cw_nb = 0;
   }
   return GMG_OK;
 }

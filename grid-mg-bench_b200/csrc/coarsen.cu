@@ -114,9 +114,10 @@ struct FineOpRef {
 };
 
 // Workspace of the construction, built on the first call and kept in the
-// aggregation: the batch size comes from the free memory then (two
+// aggregation (by the coarse-of-coarse form up to kKeptBytes): the batch size comes from the free memory then (two
 // fields of it in a third of it, at most 40 GB), the face lists and block
 // parities from the geometry.
+constexpr size_t kKeptBytes = (size_t)1 << 30;
 static gmg_status coarsen_workspace(gmg_agg* agg, cudaStream_t s) {
   if (agg->cw_nb > 0) return GMG_OK;
   const Dims& fd = agg->fdims;
@@ -269,9 +270,19 @@ gmg_status coarsen_coarse(gmg_coarse* out, gmg_agg* agg, gmg_coarse* fine, cudaS
   GMG_CHECK(fine->links_set, GMG_ERR_STATE, "coarsen: fine links not set");
   FineOpRef op;
   op.c = fine;
-  GMG_TRY(coarsen_faces(out, agg, op, s));
-  // unlike the Wilson-clover form this entry returns when the links are built
-  GMG_CUDA(cudaStreamSynchronize(s));
+  const bool had = agg->cw_nb > 0;
+  const gmg_status st = coarsen_faces(out, agg, op, s);
+  // unlike the Wilson-clover form this entry returns when the links are built, and
+  // gives a large workspace back (8^4 sites of 40 components, nbasis 40, take 0.2 GB;
+  // where it is large the construction takes far longer than the allocation)
+  const cudaError_t e = cudaStreamSynchronize(s);
+  if (!had && agg->cw_phi.bytes + agg->cw_w.bytes > kKeptBytes) {
+    agg->cw_phi.free();
+    agg->cw_w.free();
+    agg->cw_nb = 0;
+  }
+  GMG_TRY(st);
+  GMG_CUDA(e);
   return GMG_OK;
 }
 

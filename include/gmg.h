@@ -217,7 +217,7 @@ gmg_status gmg_agg_destroy(gmg_agg* h);
    one batch of right-hand sides of the fine operator (0, the default: as many
    as two fine fields of the batch in a third of the free device memory allow,
    at most 40 GB).  A smaller batch trades speed for memory; the links do not
-   depend on it.  No counterpart in the reference, which applies the fine
+   depend on it.  A change frees the workspace that the constructions keep.  No counterpart in the reference, which applies the fine
    operator to one basis vector at a time (CoarsenedMatrixUpstream.h:835-844)
    or to batches of Ls vectors, the extent of the fifth (RHS) dimension
    (...LutMRHS.h:1004-1101). */
@@ -370,9 +370,12 @@ gmg_status gmg_gauge_plaquette(const int dims[4], const double* U, int on_device
    only, and the self term as one operator pass without the hops between
    blocks of opposite parity.  The first call keeps a workspace in `agg` (two
    fine fields of a batch of basis vectors, at most 40 GB, sized from the free
-   memory then) that later calls reuse; it is freed with `agg`.  Asynchronous. */
+   memory then) that later calls reuse; it is freed with `agg` or by
+   gmg_agg_set_coarsen_batch.  Asynchronous; constructions of one `agg` on several
+   streams run one after the other. */
 gmg_status gmg_coarsen_wilson(gmg_coarse* out, gmg_agg* agg, gmg_wilson* fine, gmg_stream s);
-/* Coarse-of-coarse: the fine operator is the coarse stencil `fine`. */
+/* Coarse-of-coarse: the fine operator is the coarse stencil `fine`.  Keeps the same
+   workspace up to 1 GiB and frees a larger one again.  Synchronises the stream. */
 gmg_status gmg_coarsen_coarse(gmg_coarse* out, gmg_agg* agg, gmg_coarse* fine, gmg_stream s);
 
 /* ------------------------------------------------------------------------ */

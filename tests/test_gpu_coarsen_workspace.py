@@ -35,3 +35,41 @@ def test_constructions_on_two_streams():
         got.append((a.get_links(), b.get_links()))
     for x, y in zip(*got):
         assert np.array_equal(x, y)
+
+
+def test_large_workspace_is_given_back():
+    # two fields of 64 vectors of 12 components on 16^4 sites: 1.6 GB during the construction
+    fd, cd, dof, N = (16, 16, 16, 16), (4, 4, 4, 4), 12, 64
+    V = 65536
+    links = torch.view_as_complex(torch.randn((9, V, dof, dof, 2), dtype=torch.float64, device="cuda"))
+    fine = gmg.CoarsenedMatrix(fd, dof)
+    fine.set_links(links)
+    ag = gmg.Aggregation(fd, cd, dof, N)
+    ag.set_basis(torch.view_as_complex(torch.randn((N, V, dof, 2), dtype=torch.float64, device="cuda")))
+    out = gmg.CoarsenedMatrix(cd, N)
+    out.set_links(np.zeros((9, 256, N, N)))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    out.CoarsenOperator(ag, fine)
+    taken = free - torch.cuda.mem_get_info()[0]
+    first = out.get_links()
+    assert taken < 1 << 30, taken
+    out.CoarsenOperator(ag, fine)
+    assert np.array_equal(out.get_links(), first)
+
+
+def test_batch_change_frees_the_workspace():
+    fd, cd, N = (16, 16, 16, 16), (4, 4, 4, 4), 16
+    w = gmg.WilsonClover(fd, -0.1, 1.0, antiperiodic=1)
+    w.set_gauge(inputs.smooth_gauge(fd, inputs.rng(stream=905), 0.3))
+    ag = gmg.Aggregation(fd, cd, 12, N)
+    ag.set_basis(torch.view_as_complex(torch.randn((N, 65536, 12, 2), dtype=torch.float64, device="cuda")))
+    cm = gmg.CoarsenedMatrix(cd, N)
+    cm.CoarsenOperator(ag, w)
+    first = cm.get_links()
+    free = torch.cuda.mem_get_info()[0]
+    ag.set_coarsen_batch(4)
+    assert torch.cuda.mem_get_info()[0] - free > 300 << 20  # two fields of 201 MB
+    cm.CoarsenOperator(ag, w)
+    # other batches, other widths of the products: rounding only
+    assert np.abs(cm.get_links() - first).max() < 1e-11 * np.abs(first).max()
