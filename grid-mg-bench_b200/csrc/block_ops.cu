@@ -161,6 +161,9 @@ template <class Cx> struct ProjArgs {
 };
 
 constexpr int kProjWarps = 8;
+// blocks of so many components (a row of 4 GiB in FP64) take the kernels' forms with
+// 64-bit offsets, which need more registers per load
+constexpr int64_t kWideBlock = (int64_t)1 << 28;
 
 // The lower spin *low of (1 -+ gamma_mu) psi that is a phase (code 0: 1, 1: i, 2:
 // -1, 3: -i) times upper spin s, for hop p (p < 4: +mu, the projector 1 -
@@ -172,7 +175,8 @@ __device__ __forceinline__ int face_spin(int p, int s, int* low) {
   return (g + (p < 4 ? 2 : 0)) & 3;
 }
 
-template <class T, int MT, int RQ, bool FACE>
+// WIDE: in-block offsets in 64 bits, for blocks of 2^28 components or more
+template <class T, int MT, int RQ, bool FACE, bool WIDE = false>
 __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const ProjArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -192,9 +196,10 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
     // rows and right-hand sides past the end repeat the last one; their results are not stored
     const Cx* Vb = a.basis + c * N * K;
     const int32_t* blk = a.blk_sites + c * a.bv;
-    uint32_t row[MT];
+    typedef typename std::conditional<WIDE, uint64_t, uint32_t>::type Off;
+    Off row[MT];
     int foff[RQ];
-    const uint32_t Kb = (uint32_t)(K * sizeof(Cx));
+    const Off Kb = (Off)(K * sizeof(Cx));
 #pragma unroll
     for (int m = 0; m < MT; ++m) row[m] = min((mc * MT + m) * 8 + (lane >> 2), N - 1);
 #pragma unroll
@@ -337,9 +342,9 @@ __global__ void __launch_bounds__(32 * kProjWarps) project_mma_kernel(const Proj
   }
 }
 
-template <class T, int MT, int RQ, bool FACE>
+template <class T, int MT, int RQ, bool FACE, bool WIDE = false>
 static gmg_status launch_project(const ProjArgs<typename ctype<T>::t>& a, int Vc, cudaStream_t s) {
-  auto kern = project_mma_kernel<T, MT, RQ, FACE>;
+  auto kern = project_mma_kernel<T, MT, RQ, FACE, WIDE>;
   const size_t smem = a.KS == 1 ? 0 : sizeof(double2) * 32 * MT * RQ * (size_t)a.G * a.KS;
   if (smem > 48 * 1024)
     GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -404,14 +409,16 @@ static gmg_status project_mma(gmg_agg* h, const void* basis, int nrhs, const voi
   typedef typename ctype<T>::t Cx;
   GMG_CHECK(sizeof(Cx) * 4 * h->dof * (size_t)(h->N + nrhs) <= 227 * 1024, GMG_ERR_UNSUPPORTED,
             "project: site dof x (nbasis + nrhs) too large");
-  GMG_CHECK((int64_t)h->bv * h->dof < ((int64_t)1 << 28), GMG_ERR_UNSUPPORTED, "project: more than 2^28 components per block");
-  const int mt = (h->N + 7) / 8, mchunks = (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
+  const bool wide = (int64_t)h->bv * h->dof >= kWideBlock;
+  const int mt = (h->N + 7) / 8, mchunks = wide ? mt : (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
   const int Vc = (int)h->cdims.vol();
-  const ProjShape sh = project_shape(Vc, MT, mchunks, (nrhs + 3) / 4, FACE);
+  const ProjShape sh = wide ? ProjShape{1, (nrhs + 3) / 4, 1, kProjWarps}
+                            : project_shape(Vc, MT, mchunks, (nrhs + 3) / 4, FACE);
   const ProjArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(),
                        reinterpret_cast<const Cx*>(fine), reinterpret_cast<Cx*>(out), cstr, rstr, istr, h->N, h->dof,
                        h->bv, nrhs, sel, nsel, (int64_t)nrhs * (FACE ? 6 : h->dof), cmajor ? 1 : h->dof,
                        cmajor ? nrhs : 1, face, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
+  if (wide) return launch_project<T, 1, 1, FACE, true>(a, Vc, s);
   auto by_rq = [&](auto mtc) -> gmg_status {
     constexpr int M = decltype(mtc)::value;
     switch (sh.w) {
@@ -476,7 +483,7 @@ template <class Cx> struct PromArgs {
   int N, dof, bv, nrhs, rq;  // rq: quads of the shared-memory table
 };
 
-template <class T, int KT, int RQ>
+template <class T, int KT, int RQ, bool WIDE = false>
 __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -484,7 +491,8 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kk = lane & 3;
   const int N = a.N, dof = a.dof, steps = (N + 3) / 4;
   const int64_t c = blockIdx.x;
-  const int K = a.bv * dof;
+  typedef typename std::conditional<WIDE, int64_t, int>::type Idx;
+  const Idx K = (Idx)a.bv * dof;
   for (int e = threadIdx.x; e < steps * a.rq * 32; e += blockDim.x) {
     const int l = e & 31, q = (e >> 5) % a.rq, st = (e >> 5) / a.rq;
     const int i = 4 * st + (l & 3), r = q * 4 + (l >> 3), part = (l >> 2) & 1;
@@ -497,24 +505,26 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
   __syncthreads();
   const Cx* Vb = a.basis + c * N * (int64_t)K;
   const int32_t* blk = a.blk_sites + c * a.bv;
-  const int ngroups = (K + 8 * KT - 1) / (8 * KT), nwarps = (blockDim.x >> 5) * gridDim.y;
+  const Idx ngroups = (K + 8 * KT - 1) / (8 * KT);
+  const int nwarps = (blockDim.x >> 5) * gridDim.y;
   const int chunks = a.rq / RQ;
-  for (int item = blockIdx.y * (blockDim.x >> 5) + warp; item < ngroups * chunks; item += nwarps) {
-    const int grp = item / chunks, q0 = (item - grp * chunks) * RQ;
+  for (Idx item = blockIdx.y * (blockDim.x >> 5) + warp; item < ngroups * chunks; item += nwarps) {
+    const Idx grp = item / chunks;
+    const int q0 = (int)(item - grp * chunks) * RQ;
     double acc[KT][RQ][2];
 #pragma unroll
     for (int t = 0; t < KT; ++t)
 #pragma unroll
       for (int q = 0; q < RQ; ++q) acc[t][q][0] = acc[t][q][1] = 0.0;
-    const int k0 = grp * 8 * KT + (lane >> 2);
+    const Idx k0 = grp * 8 * KT + (lane >> 2);
     int sf[KT], at[KT];  // site and component of this lane's rows
     const Cx* Vp[KT];
 #pragma unroll
     for (int t = 0; t < KT; ++t) {
-      const int k = min(k0 + 8 * t, K - 1);
-      const int sb = k / dof;
+      const Idx k = min(k0 + 8 * t, K - 1);
+      const int sb = (int)(k / dof);
       sf[t] = blk[sb];
-      at[t] = k - sb * dof;
+      at[t] = (int)(k - (Idx)sb * dof);
       Vp[t] = Vb + k;
     }
     Cx av[2][KT];
@@ -558,17 +568,17 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
   }
 }
 
-template <class T, int KT, int RQ>
+template <class T, int KT, int RQ, bool WIDE = false>
 static gmg_status launch_promote(PromArgs<typename ctype<T>::t> a, int Vc, cudaStream_t s) {
-  auto kern = promote_mma_kernel<T, KT, RQ>;
+  auto kern = promote_mma_kernel<T, KT, RQ, WIDE>;
   const size_t smem = sizeof(double2) * 32 * (size_t)((a.N + 3) / 4) * a.rq;
   if (smem > 48 * 1024)
     GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // 8 warps per CTA; few blocks are split over several CTAs, up to 6 per SM with
   // 3 turns a warp or more (256 blocks, nbasis 32, 32 RHS: 252 us at 4, 276 at 1;
   // 16 blocks, nbasis 24, 24 RHS: 18 us at 8, 97 at 1)
-  const int items = (a.bv * a.dof + 8 * KT - 1) / (8 * KT) * (a.rq / RQ);
-  const int split = std::max(1, std::min((items + 23) / 24, (148 * 6 + Vc - 1) / Vc));
+  const int64_t items = ((int64_t)a.bv * a.dof + 8 * KT - 1) / (8 * KT) * (a.rq / RQ);
+  const int split = (int)std::max<int64_t>(1, std::min<int64_t>((items + 23) / 24, (148 * 6 + Vc - 1) / Vc));
   KernelTimer kt("promote", s);
   kern<<<dim3(Vc, split), 256, smem, s>>>(a);
   GMG_CUDA(cudaGetLastError());
@@ -581,7 +591,6 @@ static gmg_status promote_mma(gmg_agg* h, const void* basis, int nrhs, const voi
   typedef typename ctype<T>::t Cx;
   GMG_CHECK(sizeof(Cx) * ((size_t)h->N * nrhs + (size_t)h->N * 4 * h->dof) <= 227 * 1024, GMG_ERR_UNSUPPORTED,
             "promote: nbasis x (nrhs + site dof) too large");
-  GMG_CHECK((int64_t)h->bv * h->dof < ((int64_t)1 << 28), GMG_ERR_UNSUPPORTED, "promote: more than 2^28 components per block");
   // quads per warp: the fewest padded ones (each chunk reads the basis once
   // more, counted as half a quad)
   const int rq = (nrhs + 3) / 4;
@@ -596,6 +605,10 @@ static gmg_status promote_mma(gmg_agg* h, const void* basis, int nrhs, const voi
   PromArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(), reinterpret_cast<const Cx*>(coarse),
                  reinterpret_cast<Cx*>(fine), h->N, h->dof, h->bv, nrhs, w * chunks};
   const int Vc = (int)h->cdims.vol();
+  if ((int64_t)h->bv * h->dof >= kWideBlock) {
+    a.rq = rq;
+    return launch_promote<T, 4, 1, true>(a, Vc, s);
+  }
   switch (w) {
     case 1: return launch_promote<T, 4, 1>(a, Vc, s);
     case 2: return launch_promote<T, 4, 2>(a, Vc, s);
