@@ -176,11 +176,15 @@ namespace gmg {
 typedef std::array<int64_t, 7> TuneKey;
 bool tuned_find(const TuneKey& key, uint32_t* choice);
 // what a Wilson-clover variant is chosen by: vector precision, fused products or not,
-// single-hop op or not, nrhs class, alignment class of the fields (0: 32 bytes, 1: 16, 2: less)
-inline uint64_t wilson_tune_key(int vec_prec, bool dots, bool single_hop, int nrhs, int align) {
-  const int cls = nrhs < 4 ? 0 : nrhs < 8 ? 1 : nrhs < 16 ? 2 : nrhs < 32 ? 3 : 4;
-  return (uint64_t)vec_prec | ((uint64_t)dots << 4) | ((uint64_t)single_hop << 5) | ((uint64_t)align << 6) |
-         ((uint64_t)cls << 8);
+// kind of operator (0: M, Mdag, 1: a single hop, 2: Mdiag), nrhs class, alignment class
+// of the fields (0: 32 bytes, 1: 16, 2: less).  One right-hand side is a class of its own,
+// as Mdiag is a kind: the site kernel wins these by far more than their neighbours, where it
+// may lose (FP64 M 8^4, site / tile kernel: 1 right-hand side 8.3 / 8.3 us, 2 12.4 / 10.3; FP32
+// 16^4 x 4, Mdiag 16 / 25, M 56 / 41).
+inline uint64_t wilson_tune_key(int vec_prec, bool dots, int op, int nrhs, int align) {
+  const int cls = nrhs < 2 ? 0 : nrhs < 4 ? 1 : nrhs < 8 ? 2 : nrhs < 16 ? 3 : nrhs < 32 ? 4 : 5;
+  return (uint64_t)vec_prec | ((uint64_t)dots << 4) | ((uint64_t)op << 5) | ((uint64_t)align << 7) |
+         ((uint64_t)cls << 9);
 }
 void tuned_store(const TuneKey& key, uint32_t choice);
 

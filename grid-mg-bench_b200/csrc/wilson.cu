@@ -1775,10 +1775,10 @@ static gmg_status run_variant(gmg_wilson* h, int v, bool dots, int op, int dir, 
 }
 
 // Autotuned dispatch.  The kernel variant is chosen per (vector precision,
-// fused products or not, single-hop op or not, nrhs class) by timing every
-// applicable variant once on the call that first meets the key (CUDA events
+// fused products or not, kind of operator, nrhs class, alignment of the fields) by
+// timing the variants that can win there once on the call that first meets the key (CUDA events
 // on the caller's stream; not while the stream is being captured) and is
-// cached in the handle.  The nrhs classes (1-3, 4-7, 8-15, 16-31, 32+) keep a
+// cached in the handle.  The nrhs classes (1, 2-3, 4-7, 8-15, 16-31, 32+) keep a
 // batch that shrinks as right-hand sides converge from re-tuning at every size.
 static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int disp, int vec_prec, int nrhs,
                                   const void* in, void* out, double2* d1, double2* d2, cudaStream_t s) {
@@ -1798,7 +1798,8 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
   }
   // fields of lesser alignment, which some variants refuse, are timed on their own
   const uintptr_t al = (uintptr_t)in | (uintptr_t)out;
-  const uint64_t key = wilson_tune_key(vec_prec, dots, op == GMG_OP_MDIR, nrhs, al & 15 ? 2 : al & 31 ? 1 : 0);
+  const int opc = op == GMG_OP_MDIR ? 1 : op == GMG_OP_MDIAG ? 2 : 0;
+  const uint64_t key = wilson_tune_key(vec_prec, dots, opc, nrhs, al & 15 ? 2 : al & 31 ? 1 : 0);
   auto it = h->wtune.find(key);
   // the choice of an earlier handle on the same lattice
   TuneKey shared = {};
@@ -1821,11 +1822,14 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     cand.push_back(kTileOcc3);
     cand.push_back(kTileOcc3Pf);
   }
-  // the quad and staged kernels run when forced, the quad kernel also where the
-  // others do not apply (fields below 16-byte alignment); timing them on first calls
-  // found no key they win (8^4 to 32^4, 1 to 24 right-hand sides, both precisions)
-  // and took up to two thirds of such a call
-  if (((uintptr_t)in | (uintptr_t)out) & 15) cand.push_back(GMG_WILSON_QUAD);
+  // the staged kernel on lattices that leave most of the chip idle, where its two roles
+  // and its bulk copies shorten the chain of one site (FP64 M, staged / tile kernel, us:
+  // 4^4 x 4 right-hand sides 6.2 / 8.3, x 24 8.3 / 18.5; 8^3 x 16, 16: 37 / 42; FP32 4^3 x 8,
+  // 24: 6.2 / 8.3; from 12^4 on it wins nowhere, and timing it took up to two thirds of a
+  // first call); the quad kernel where the others do not apply (fields below 16-byte
+  // alignment).  Elsewhere both run when forced.
+  if (nrhs >= 4 && h->dims.vol() <= 8192) cand.push_back(GMG_WILSON_STAGED);
+  if (al & 15) cand.push_back(GMG_WILSON_QUAD);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GMG_CUDA(cudaStreamIsCapturing(s, &cap));
   int best = nrhs >= 4 ? GMG_WILSON_TILE : (dots ? GMG_WILSON_QUAD : GMG_WILSON_SITE);

@@ -294,10 +294,13 @@ gmg_status gmg_wilson_apply_f32_in(gmg_wilson* h, gmg_op op, int nrhs, const flo
    in the low 16 bits), FP32 arithmetic, the products from the FP32 result,
    the result rounded to nearest even (the fine smoother of params.smoother_bf16). */
 /* Kernel variants of the multi-RHS Wilson-clover apply.  By default the
-   variant is autotuned: every applicable one is timed once per (vector
-   precision, fused MR products or not, single-hop op or not, nrhs class) on
-   the first call in the process that meets the key on a lattice, and the fastest
-   is kept in the handle and for later handles of the same lattice.
+   variant is autotuned: those that can win are timed once per (vector
+   precision, fused MR products or not, kind of op (M and Mdag, Mdiag, one hop),
+   nrhs class, alignment of the fields) on the first call in the process that meets
+   the key on a lattice, and the fastest is kept in the handle and for later handles
+   of the same lattice.  SITE is timed for fewer than 8 right-hand sides without
+   products, STAGED for 4 or more on up to 8192 sites, QUAD for fields below 16-byte
+   alignment.
    gmg_wilson_set_kernel forces one (GMG_WILSON_AUTO restores tuning); a forced
    variant that does not apply to a call falls back to the tuned choice. */
 typedef enum {

@@ -126,3 +126,22 @@ def test_choices_by_alignment():
     assert w.tuned_kernel("f32", 12) == "quad"
     w.M(x, torch.zeros_like(x))
     assert w.tuned_kernel("f32", 12) == "tile"
+
+
+def test_choices_by_kind_of_operator():
+    # the site kernel wins Mdiag by far more than M: one's choice is not the other's
+    dims = (16, 16, 16, 16)
+    x = _field("f32", 6, 883, 65536)
+    out = torch.zeros_like(x)
+    w = _handle(884, None, dims)
+    w.Mdiag(x, out)
+    assert w.tuned_kernel("f32", 6) == "auto"  # M's, not timed yet
+    w.M(x, out)
+    assert w.tuned_kernel("f32", 6) == "tile"
+
+
+def test_small_lattice_times_the_staged_kernel():
+    x = _field("f64", 12, 885, 256)
+    w = _handle(886, None, (4, 4, 4, 4))
+    w.M(x, torch.zeros_like(x))
+    assert w.tuned_kernel("f64", 12) == "staged"
