@@ -1816,8 +1816,8 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
     if (launched) return GMG_OK;
   }
   std::vector<int> cand;
-  if (!dots && nrhs < 8) cand.push_back(GMG_WILSON_SITE);
   cand.push_back(GMG_WILSON_TILE);
+  if (!dots && nrhs < 8) cand.push_back(GMG_WILSON_SITE);
   if (vec_prec == GMG_F32) {
     cand.push_back(kTileOcc3);
     cand.push_back(kTileOcc3Pf);
@@ -1845,13 +1845,23 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
       st = run_variant(h, v, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &ok);  // warm-up
       if (st != GMG_OK) break;
       if (!ok) continue;
-      if (cudaEventRecord(e0, s) != cudaSuccess) break;
-      for (int k = 0; k < 2 && st == GMG_OK; ++k)
-        st = run_variant(h, v, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &ok);
-      if (st != GMG_OK || cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) break;
+      // two launches, or ten where those take less than 50 us (a launch's own jitter
+      // decided between variants there); a later variant has to be 2 % faster
       float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best_ms) {
+      for (int n = 2; n <= 10; n += 8) {
+        if (cudaEventRecord(e0, s) != cudaSuccess) break;
+        for (int k = 0; k < n && st == GMG_OK; ++k)
+          st = run_variant(h, v, dots, op, dir, disp, vec_prec, nrhs, in, out, d1, d2, s, &ok);
+        if (st != GMG_OK || cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+            cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
+          ms = 0.f;
+          break;
+        }
+        ms /= n;
+        if (ms > 0.025f) break;
+      }
+      if (st != GMG_OK || ms == 0.f) break;
+      if (ms < 0.98f * best_ms) {
         best_ms = ms;
         best = v;
       }
