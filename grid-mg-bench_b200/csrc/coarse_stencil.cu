@@ -17,6 +17,7 @@
 // Links are kept site-major, [V][9][N][N], so that one site's 9 matrices are
 // one contiguous stream.
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "f64_mma.cuh"
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(mma_threads(MT * RQ)) coarse_mma_kernel(const 
     const int npts = a.p1 - a.p0;
     unsigned pts = ((1u << (a.p0 + (ks + 1) * npts / a.KS)) - 1) & ~((1u << (a.p0 + ks * npts / a.KS)) - 1);
     if (a.skip) pts &= ~(unsigned)a.skip[site];
-    // Both operands are requested two steps ahead of their use, into the other
+    // Both operands are requested one step ahead of their use, into the other
     // of two register sets.
     if (pts) {
       C av[2][MT], fv[2][RQ];
@@ -283,30 +284,83 @@ static gmg_status launch_mma(const MmaArgs<typename cplx_t<T>::type>& a, int nsi
   return GMG_OK;
 }
 
+// Registers a thread of coarse_mma_kernel<T, MT, RQ> (allocated in eights; nvcc
+// 12.9), which decide how many warps an SM holds.  A wrong entry costs speed only.
+static int mma_regs(bool f64, int MT, int w) {
+  static const unsigned char tab[2][5][5] = {{
+      {56, 72, 72, 88, 96},
+      {72, 80, 96, 112, 128},
+      {72, 96, 128, 128, 152},
+      {88, 112, 128, 160, 176},
+      {96, 128, 160, 192, 208}}, {
+      {64, 72, 96, 96, 120},
+      {72, 96, 112, 128, 152},
+      {96, 120, 128, 160, 184},
+      {112, 136, 160, 192, 216},
+      {128, 160, 192, 224, 248}}};
+  return tab[f64 ? 1 : 0][MT - 1][w - 1];
+}
+
 // Launch shape: quads of right-hand sides per unit (w, in `chunks` chunks),
-// units (G) and point shares (KS) per CTA.  w gives the fewest padded quads
-// (each chunk reads the links once more, counted as half a quad).  One warp per
-// unit is fastest where the lattice fills the chip (4096 sites, nbasis 32, 32 RHS, FP64:
-// 356 us, 431 with two shares); below that the points are split until
-// every SM has about 12 warps, or 24 of the small tiles, whose steps are too
-// short to hide the operands' latency (840 sites, nbasis 40, 5 RHS, FP32: 39 us
-// with 5 shares, 44 with 2, 48 with 1).
+// units (G) and point shares (KS) per CTA.
+// w gives the fewest padded quads (each chunk reads the links once more, counted
+// as half a quad).  FP32 from 7 quads on: where the registers of a tile leave fewer
+// than 14 warps per SM its operands' latency shows, and a narrower tile wins (4096
+// sites, nbasis 34, 48 RHS: 936 us with w = 4, 714 with 3).  A single point, which
+// cannot be split, takes narrower tiles until every scheduler has a warp.
+// G: all the units that fit, or half of them or one where that puts a third more
+// warps on an SM (FP32, nbasis 50, 64 RHS, 4096 sites: 8 units a CTA 2603 us, 4 2110).
+// KS: one warp per unit is fastest where the lattice fills the chip (4096 sites,
+// nbasis 32, 32 RHS, FP64: 356 us, 431 with two shares); below that the points are
+// split until every SM has about 12 warps, or 24 of the small tiles, whose steps are
+// too short to hide the operands' latency (840 sites, nbasis 40, 5 RHS, FP32: 39 us
+// with 5 shares, 44 with 2, 48 with 1).  A split of big tiles, or into 5 or 9 shares,
+// that would turn one wave of CTAs into one and up to a half is not made (256 sites,
+// nbasis 32, 32 RHS, FP64: 5 shares 50 us, 2 31 us).
 struct MmaShape {
   int w, chunks, G, KS;
 };
-static MmaShape mma_shape(int64_t nsites, int npts, int MT, int mchunks, int rq) {
+static MmaShape mma_shape(bool f64, int64_t nsites, int npts, int MT, int mchunks, int rq) {
   MmaShape sh{1, rq, 1, 1};
-  for (int w = 2; w <= 5; ++w) {
-    const int u = (rq + w - 1) / w;
-    if (u * (2 * w + 1) <= sh.chunks * (2 * sh.w + 1)) sh = MmaShape{w, u, 1, 1};
+  double best = 1e30;
+  for (int w = 1; w <= std::min(5, rq); ++w) {
+    const int u = (rq + w - 1) / w, warps = 65536 / (32 * mma_regs(f64, MT, w));
+    double cost = u * (2 * w + 1);
+    if (!f64 && rq >= 7 && warps < 14) cost *= std::pow(14.0 / warps, 0.6);
+    if (cost <= best) {
+      best = cost;
+      sh = MmaShape{w, u, 1, 1};
+    }
   }
-  const int units = mchunks * sh.chunks, maxw = mma_threads(MT * sh.w) / 32;
+  while (npts == 1 && sh.w > 1 && nsites * mchunks * sh.chunks < 148 * 4) {
+    sh.w = (sh.w + 1) / 2;
+    sh.chunks = (rq + sh.w - 1) / sh.w;
+  }
+  const int units = mchunks * sh.chunks, maxw = mma_threads(MT * sh.w) / 32, regs = mma_regs(f64, MT, sh.w);
   const int64_t want = 148 * (MT * sh.w > 10 ? 12 : 24);
+  int64_t wave = 0;  // CTAs of the split before, where those fit the chip at once
   for (const int ks : {1, 2, 3, 5, 9}) {
-    sh.KS = std::min(ks, std::min(npts, maxw));
-    if (nsites * units * sh.KS >= want) break;
+    const int KS = std::min(ks, std::min(npts, maxw)), gmax = std::min(units, maxw / KS);
+    int G = 0;
+    int64_t ctas = 0, slots = 0;
+    double most = 0.0;
+    for (const int g : {gmax, std::max(1, maxw / KS / 2), 1}) {
+      if (g > gmax) continue;
+      const int per = (units + g - 1) / g;
+      const int64_t q = nsites * per, C = std::max(1, std::min(65536 / (32 * regs * g * KS), std::min(64 / (g * KS), 32)));
+      const double warps = (double)std::min(C, (q + 147) / 148) * g * KS * units / (per * g);
+      if (G == gmax ? warps < 1.3 * most : G && warps <= most) continue;
+      G = g;
+      most = warps;
+      ctas = q;
+      slots = 148 * C;
+    }
+    if ((MT * sh.w > 10 || ks >= 5) && wave && ctas > slots && ctas < slots * 3 / 2) break;
+    wave = ctas <= slots ? ctas : 0;
+    sh.KS = KS;
+    sh.G = G;
+    if (nsites * units * KS >= want) break;
   }
-  sh.G = std::min(units, maxw / sh.KS);
   return sh;
 }
 
@@ -318,7 +372,7 @@ static gmg_status coarse_mma(const LinkSel& L, const void* in, void* out, int V,
   const int mt = (N + 7) / 8, mchunks = (mt + 4) / 5, MT = (mt + mchunks - 1) / mchunks;
   const int nsites = sel ? nsel : V, npts = p1 - p0;
   if (nsites == 0) return GMG_OK;
-  const MmaShape sh = mma_shape(nsites, npts, MT, mchunks, (R + 3) / 4);
+  const MmaShape sh = mma_shape(sizeof(T) == 8, nsites, npts, MT, mchunks, (R + 3) / 4);
   MmaArgs<C> a{reinterpret_cast<const C*>(L.links), L.link_pts, L.pbase, L.site_map, L.nbr, L.dag,
                reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), V, N, nrhs, active, R, p0, p1, g5,
                sel, skip, mchunks * sh.chunks, sh.chunks, sh.G, sh.KS};
