@@ -481,9 +481,11 @@ template <class Cx> struct PromArgs {
   const Cx* coarse;
   Cx* fine;
   int N, dof, bv, nrhs, rq;  // rq: quads of the shared-memory table
+  int rlim;                  // right-hand sides from `coarse` and `fine` on (nrhs: their stride)
 };
 
-template <class T, int KT, int RQ, bool WIDE = false>
+// PART: a part of the right-hand sides, the first a.rlim from a.coarse and a.fine on
+template <class T, int KT, int RQ, bool WIDE = false, bool PART = false>
 __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typename ctype<T>::t> a) {
   typedef typename ctype<T>::t Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
     const int l = e & 31, q = (e >> 5) % a.rq, st = (e >> 5) / a.rq;
     const int i = 4 * st + (l & 3), r = q * 4 + (l >> 3), part = (l >> 2) & 1;
     Cx v{0, 0};
-    if (i < N && r < a.nrhs) v = a.coarse[(c * a.nrhs + r) * N + i];
+    if (i < N && r < (PART ? a.rlim : a.nrhs)) v = a.coarse[(c * a.nrhs + r) * N + i];
     double2 b;
     f64mma::expand(v, part, 0u, f64mma::second_sign(part, false), b.x, b.y);
     Bs[e] = b;
@@ -558,7 +560,7 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
 #pragma unroll
       for (int q = 0; q < RQ; ++q) {
         const int r = (q0 + q) * 4 + kk;
-        if (r >= a.nrhs) continue;
+        if (r >= (PART ? a.rlim : a.nrhs)) continue;
         Cx v;
         v.x = acc[t][q][0];
         v.y = acc[t][q][1];
@@ -568,19 +570,44 @@ __global__ void __launch_bounds__(256) promote_mma_kernel(const PromArgs<typenam
   }
 }
 
-template <class T, int KT, int RQ, bool WIDE = false>
+template <class T, int KT, int RQ, bool WIDE = false, bool PART = false>
 static gmg_status launch_promote(PromArgs<typename ctype<T>::t> a, int Vc, cudaStream_t s) {
-  auto kern = promote_mma_kernel<T, KT, RQ, WIDE>;
+  auto kern = promote_mma_kernel<T, KT, RQ, WIDE, PART>;
+  const int launches = PART ? a.rq / RQ : 1;  // PART: a chunk of right-hand sides each
+  if (PART) a.rq = RQ;
   const size_t smem = sizeof(double2) * 32 * (size_t)((a.N + 3) / 4) * a.rq;
   if (smem > 48 * 1024)
     GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // 8 warps per CTA; few blocks are split over several CTAs, up to 6 per SM with
   // 3 turns a warp or more (256 blocks, nbasis 32, 32 RHS: 252 us at 4, 276 at 1;
-  // 16 blocks, nbasis 24, 24 RHS: 18 us at 8, 97 at 1)
+  // 16 blocks, nbasis 24, 24 RHS: 18 us at 8, 97 at 1).  A block with no more than one
+  // item a warp takes CTAs of fewer warps where that keeps more of them busy and on an
+  // SM, which then overlap each other's tables and ends (4096 blocks of 2^4 x 12, nbasis
+  // 16, 16 RHS, FP32: 180 us with 8, 97 with 2; FP64 nbasis 2, 1 RHS: 24 and 15).
   const int64_t items = ((int64_t)a.bv * a.dof + 8 * KT - 1) / (8 * KT) * (a.rq / RQ);
-  const int split = (int)std::max<int64_t>(1, std::min<int64_t>((items + 23) / 24, (148 * 6 + Vc - 1) / Vc));
+  int nw = 8;
+  if (items <= 8) {
+    // registers a thread, as compiled by nvcc 12.9 (a wrong entry costs speed only)
+    static const int tab[2][8] = {{88, 112, 128, 144, 128, 112, 120, 120}, {80, 104, 128, 144, 128, 104, 120, 120}};
+    const int regs = tab[sizeof(T) == 8 ? 0 : 1][RQ - 1];
+    double most = 0.0;
+    for (const int n : {8, 6, 4, 3, 2}) {
+      const int64_t C = std::max<int64_t>(1, std::min<int64_t>(65536 / (32 * regs * n), 227 * 1024 / (smem + 1024)));
+      const double busy = (double)std::min<int64_t>(C, (Vc + 147) / 148) * items / ((items + n - 1) / n);
+      if (busy > 1.2 * most) {
+        most = busy;
+        nw = n;
+      }
+    }
+  }
+  const int split = (int)std::max<int64_t>(1, std::min<int64_t>((items + 3 * nw - 1) / (3 * nw), (148 * 48 / nw + Vc - 1) / Vc));
   KernelTimer kt("promote", s);
-  kern<<<dim3(Vc, split), 256, smem, s>>>(a);
+  for (int k = 0; k < launches; ++k) {
+    kern<<<dim3(Vc, split), 32 * nw, smem, s>>>(a);
+    a.coarse += (int64_t)4 * RQ * a.N;
+    a.fine += (int64_t)4 * RQ * a.dof;
+    a.rlim -= 4 * RQ;
+  }
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
@@ -603,12 +630,17 @@ static gmg_status promote_mma(gmg_agg* h, const void* basis, int nrhs, const voi
     }
   }
   PromArgs<Cx> a{reinterpret_cast<const Cx*>(basis), h->blk_sites.as<int32_t>(), reinterpret_cast<const Cx*>(coarse),
-                 reinterpret_cast<Cx*>(fine), h->N, h->dof, h->bv, nrhs, w * chunks};
+                 reinterpret_cast<Cx*>(fine), h->N, h->dof, h->bv, nrhs, w * chunks, nrhs};
   const int Vc = (int)h->cdims.vol();
   if ((int64_t)h->bv * h->dof >= kWideBlock) {
     a.rq = rq;
     return launch_promote<T, 4, 1, true>(a, Vc, s);
   }
+  // a table that leaves room for one CTA on an SM only (nbasis above 56, 57 right-hand
+  // sides and more) is made by chunk, one launch each, where blocks enough for both wait
+  // (4096 blocks of 2^4 x 12, nbasis 64, 64 RHS, FP32: 1490 us with all of it, 1070)
+  if (Vc >= 148 * 2 && sizeof(double2) * 32 * (size_t)((h->N + 3) / 4) * a.rq > 112 * 1024)
+    return w == 5 ? launch_promote<T, 3, 5, false, true>(a, Vc, s) : launch_promote<T, 2, 8, false, true>(a, Vc, s);
   switch (w) {
     case 1: return launch_promote<T, 4, 1>(a, Vc, s);
     case 2: return launch_promote<T, 4, 2>(a, Vc, s);
