@@ -54,9 +54,10 @@ gmg_status agg_build_tables(gmg_agg* h, cudaStream_t s) {
 // basis [i][site][dof] <-> basis_blk [c][i][sb*dof + a].  Bound by HBM, both sides
 // once.  A thread keeps one (c, sb*dof + a), whose place in either layout it works
 // out once, and walks basis vectors blockIdx.y, + gridDim.y, ..., eight requests at
-// a time: 32^4 x 12, nbasis 32, 2.32 -> 1.94 ms in and 2.28 -> 2.00 ms back, 6.4 to
-// 6.6 TB/s, against one element a thread and step with its divisions.
-template <bool TO_BLK>
+// a time (U; one where a thread has few): 32^4 x 12, nbasis 32, 2.32 -> 1.94 ms in and
+// 2.28 -> 2.00 ms back, 6.4 to 6.6 TB/s, against one element a thread and step with its
+// divisions.
+template <bool TO_BLK, int U>
 __global__ void __launch_bounds__(256) basis_layout_kernel(const double2* __restrict__ src, double2* __restrict__ dst,
                                                            const int32_t* __restrict__ blk_sites, int64_t Vc, int N,
                                                            int bv, int dof, int64_t Vf) {
@@ -67,7 +68,6 @@ __global__ void __launch_bounds__(256) basis_layout_kernel(const double2* __rest
   const double2* in = src + (TO_BLK ? nat : blk);
   double2* out = dst + (TO_BLK ? blk : nat);
   const int64_t si = TO_BLK ? Vf * dof : K, so = TO_BLK ? K : Vf * dof;
-  constexpr int U = 8;
   for (int i0 = blockIdx.y; i0 < N; i0 += U * gridDim.y) {
     double2 v[U];
 #pragma unroll
@@ -82,11 +82,15 @@ __global__ void __launch_bounds__(256) basis_layout_kernel(const double2* __rest
 template <bool TO_BLK>
 static gmg_status basis_layout(gmg_agg* h, const double2* src, double2* dst, cudaStream_t s) {
   const int64_t Vc = h->cdims.vol(), n = (Vc * h->bv * h->dof + 255) / 256;
-  // the basis vectors split over CTAs only while those do not fill the chip
-  const int split = (int)std::max<int64_t>(1, std::min<int64_t>((h->N + 7) / 8, 148 * 8 / n));
+  // the basis vectors split over CTAs only while those do not fill the chip (256 sites x
+  // 12, nbasis 8, out: 4.1 us by one CTA per 256 elements, 3.5 by eight)
+  const int64_t most = std::max<int64_t>(1, 148 * 8 / n);
+  int split = (int)std::min<int64_t>((h->N + 7) / 8, most);
+  if (n * split < 148 * 2) split = (int)std::min<int64_t>(h->N, most);
   GMG_CHECK(n < ((int64_t)1 << 31), GMG_ERR_UNSUPPORTED, "basis layout: lattice too large");
-  basis_layout_kernel<TO_BLK><<<dim3((unsigned)n, split), 256, 0, s>>>(src, dst, h->blk_sites.as<int32_t>(), Vc, h->N,
-                                                                       h->bv, h->dof, h->fdims.vol());
+  auto kern = h->N < 4 * split ? basis_layout_kernel<TO_BLK, 1> : basis_layout_kernel<TO_BLK, 8>;
+  kern<<<dim3((unsigned)n, split), 256, 0, s>>>(src, dst, h->blk_sites.as<int32_t>(), Vc, h->N, h->bv, h->dof,
+                                                h->fdims.vol());
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }

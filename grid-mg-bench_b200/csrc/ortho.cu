@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(NT > 4 ? 256 : 384) gram_kernel(Params P) {
       gr += d[at];
       gi += X == Y ? d[64 + at] - d[64 + mirror] : d[64 + at];
     }
-    if (i == j) gi = 0.0;  // also where both terms overflowed
+    if (CHECK && i == j) gi = 0.0;  // also where both terms overflowed (the factor takes real diagonals)
     if (CHECK) {
       const double x = gr - (i == j ? 1.0 : 0.0);
       mx = fmax(mx, sqrt(x * x + gi * gi));
