@@ -80,11 +80,11 @@ def build(force=False, verbose_ptxas=False, jobs=None):
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
         relinked = True
-    # host programs over the C++ surface (include/gmg.hpp), linked against the library
+    # host programs over the C++ surface (include/gmg.hpp) and over internal entry points, linked against the library
     for src in sorted(glob.glob(os.path.join(HERE, "host", "*.cpp"))):
         exe = os.path.join(BUILD, os.path.basename(src)[:-4])
         if force or relinked or _stale(src, exe, hdr_mtime):
-            cmd = [cc, "-O2", "-std=c++17", "-I", INCLUDE, src, "-o", exe, "-L", HERE, "-lgmg_b200",
+            cmd = [cc, "-O2", "-std=c++17", "-I", INCLUDE, "-I", CSRC, src, "-o", exe, "-L", HERE, "-lgmg_b200",
                    "-Xlinker", "-rpath=$ORIGIN/..", "-lcudart"]
             r = subprocess.run(cmd, capture_output=True, text=True)
             if r.returncode != 0:
