@@ -405,10 +405,6 @@ static gmg_status coarse_mma(const LinkSel& L, const void* in, void* out, int V,
 // shared-memory tiles (row stride N + 1 complex numbers: no bank conflicts).
 // Needs TB | N and TR | R.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async_c(void* dst, const double2* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_c(void* dst, const float2* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");

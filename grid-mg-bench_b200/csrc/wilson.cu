@@ -471,7 +471,8 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
 // The backward hops read U_mu(x - mu) of the neighbour's run.  Per site and RHS
 // that is 1536 bytes in FP64, against 2112 for the site-major arrays, whose
 // 16-byte reads at 576- and 1152-byte strides also took a line each.  32^4, one
-// RHS: FP64 847 -> 380 us (1.6 GB, 4.2 TB/s; 390 and 575 us at 4 and 5 CTAs per SM,
+// RHS: FP64 847 -> 380 to 420 us by machine (1.6 GB, 3.8 to 4.2 TB/s; where it takes
+// 380, 390 and 575 us at 4 and 5 CTAs per SM,
 // which spill), FP32 497 -> 168 us (189 at 4 CTAs per SM).
 constexpr int kSoa = 32, kSoaThreads = 128;
 
@@ -1897,7 +1898,7 @@ static gmg_status wilson_dispatch(gmg_wilson* h, bool dots, int op, int dir, int
 // Half of Mdir_p on nq listed in-block sites `sel` of every block: out[(c * nq +
 // q)][6][nrhs] = coef U (upper two spins of (1 -+ gamma_mu) psi(neighbour)).  The
 // lower two spins are fixed combinations of the upper ones, so the face
-// projections need these six components only (see project_half_kernel).
+// projections need these six components only (project_mma_kernel's FACE form).
 __global__ void __launch_bounds__(256) wilson_face_half_kernel(
     const double2* __restrict__ hop, const int32_t* __restrict__ nbr, const double2* __restrict__ in,
     double2* __restrict__ out, const int32_t* __restrict__ blk_sites, const int32_t* __restrict__ sel, int nq, int bv,
