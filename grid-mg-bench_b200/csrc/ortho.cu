@@ -84,6 +84,7 @@ struct Params {
   unsigned long long* maxerr;  // check mode: max |G - 1| (as the bits of a non-negative double)
   int Vc, N, K;
   int pass, passes;
+  int whole;  // the wide substitution's CTAs take whole blocks
 };
 
 __device__ __forceinline__ bool block_active(const Params& P, int c) { return P.pass < P.passes || P.need[c] != 0; }
@@ -296,18 +297,8 @@ __device__ __forceinline__ void tri_solve_body(const Params& P) {
   const int N = EXACT ? NMAX : P.N, K = P.K, t = threadIdx.x;
   const int nl = N * (N + 1) / 2;
   const int chunks = (K + NTS - 1) / NTS;
-  // this CTA's items: n (block c, chunk ch) pairs in order from its first; inactive blocks are passed over
-  const int64_t total = (int64_t)P.Vc * chunks, per = (total + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
-  int n = (int)max((int64_t)0, min(per, total - first)), c = (int)(first / chunks), ch = (int)(first % chunks);
-  auto skip = [&](int& n, int& c, int& ch) {
-    while (n > 0 && !block_active(P, c)) {
-      n -= chunks - ch;
-      ++c;
-      ch = 0;
-    }
-  };
-  auto prefetch = [&](int n, int c, int ch) {
-    const int k = n > 0 ? ch * NTS + t : K;
+  auto prefetch = [&](bool valid, int c, int ch) {
+    const int k = valid ? ch * NTS + t : K;
     if (k < K) {
       const double2* col = P.basis + (int64_t)c * N * K + k;
 #pragma unroll
@@ -317,16 +308,7 @@ __device__ __forceinline__ void tri_solve_body(const Params& P) {
     cp_async_commit();
   };
   int lc = -1;  // the block whose factor is in L
-  skip(n, c, ch);
-  prefetch(n, c, ch);
-  while (n > 0) {
-    // the item after this one
-    int nn = n - 1, nc = c, nch = ch + 1;
-    if (nch == chunks) {
-      ++nc;
-      nch = 0;
-    }
-    skip(nn, nc, nch);
+  auto item = [&](int c, int ch, auto prefetch_next) {
     if (c != lc) {
       __syncthreads();  // every thread is done with the previous block's factor
       const double2* src = P.lfac + (int64_t)c * nl;
@@ -339,7 +321,7 @@ __device__ __forceinline__ void tri_solve_body(const Params& P) {
     double2 w[NMAX];
 #pragma unroll
     for (int i = 0; i < NMAX; ++i) w[i] = (i < N && k < K) ? pre[i * NTS + t] : make_double2(0.0, 0.0);
-    prefetch(nn, nc, nch);  // the slots are free again: copy the next item's columns meanwhile
+    prefetch_next();  // the slots are free again: copy the next item's columns meanwhile
     if (k < K) {
       // rows in groups of four: the products with the already solved entries
       // (j below the group) are independent across the group's rows, two
@@ -394,9 +376,55 @@ __device__ __forceinline__ void tri_solve_body(const Params& P) {
       for (int i = 0; i < NMAX; ++i)
         if (i < N) col[(int64_t)i * K] = w[i];
     }
-    n = nn;
-    c = nc;
-    ch = nch;
+  };
+  if constexpr (NMAX > 32) {
+    // items [it, end): chunk it % chunks of block(it / chunks), a run of all blocks' chunks or
+    // whole blocks at the grid's stride.  One index and a division per item: the state of
+    // the loop below slowed these instances, whose column alone takes 160 registers (433
+    // -> 375 us at 4096 blocks of 192 columns, nbasis 36)
+    const int total = P.Vc * chunks, per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
+    int it = P.whole ? 0 : min((int)blockIdx.x * per, total);
+    const int end = P.whole ? (P.Vc - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * chunks : min(it + per, total);
+    auto block = [&](int q) { return P.whole ? (int)blockIdx.x + q * (int)gridDim.x : q; };
+    auto active_from = [&](int i) {
+      while (i < end && !block_active(P, block(i / chunks))) i = (i / chunks + 1) * chunks;
+      return i;
+    };
+    it = active_from(it);
+    prefetch(it < end, block(it / chunks), it % chunks);
+    while (it < end) {
+      const int q = it / chunks;
+      item(block(q), it - q * chunks, [&] {
+        it = active_from(it + 1);
+        prefetch(it < end, block(it / chunks), it % chunks);
+      });
+    }
+  } else {
+    // this CTA's items: n (block c, chunk ch) pairs in order from its first; inactive blocks are passed over
+    const int64_t total = (int64_t)P.Vc * chunks, per = (total + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
+    int n = (int)max((int64_t)0, min(per, total - first)), c = (int)(first / chunks), ch = (int)(first % chunks);
+    auto skip = [&](int& n, int& c, int& ch) {
+      while (n > 0 && !block_active(P, c)) {
+        n -= chunks - ch;
+        ++c;
+        ch = 0;
+      }
+    };
+    skip(n, c, ch);
+    prefetch(n > 0, c, ch);
+    while (n > 0) {
+      // the item after this one
+      int nn = n - 1, nc = c, nch = ch + 1;
+      if (nch == chunks) {
+        ++nc;
+        nch = 0;
+      }
+      skip(nn, nc, nch);
+      item(c, ch, [&] { prefetch(nn > 0, nc, nch); });
+      n = nn;
+      c = nc;
+      ch = nch;
+    }
   }
   cp_async_wait<0>();
 }
@@ -620,6 +648,7 @@ static gmg_status workspace(gmg_agg* h, Params* P) {
   P->N = h->N;
   P->K = h->bv * h->dof;
   P->pass = 0;
+  P->whole = 0;
   P->passes = 1;
   return GMG_OK;
 }
@@ -669,9 +698,17 @@ static gmg_status launch_solve(const Params& P, cudaStream_t s) {
   GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 1;
   GMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSolveThreads, smem));
-  const int64_t items = (int64_t)P.Vc * ((P.K + kSolveThreads - 1) / kSolveThreads);
-  const int grid = (int)std::min<int64_t>(items, num_sms() * std::max(per_sm, 1));
-  kern<<<grid, kSolveThreads, smem, s>>>(P);
+  const int64_t chunks = (P.K + kSolveThreads - 1) / kSolveThreads, items = P.Vc * chunks;
+  const int64_t slots = num_sms() * std::max(per_sm, 1), by_block = std::min<int64_t>(P.Vc, slots);
+  int64_t grid = std::min<int64_t>(items, slots);
+  // nbasis above 32: whole blocks at the grid's stride, whose CTAs walk the rows side by side, unless that
+  // takes a CTA a fifth more chunks than equal runs of them (24^4, 1296 blocks of 4^4,
+  // nbasis 40: 1509 us, in runs 1705; 16^4, 256 blocks, nbasis 32: 220, in runs 200; 81
+  // blocks, nbasis 40: 195, in runs 113)
+  Params Q = P;
+  Q.whole = NMAX > 32 && 5 * ((P.Vc + by_block - 1) / by_block * chunks) <= 6 * ((items + grid - 1) / grid);
+  if (Q.whole) grid = by_block;
+  kern<<<(int)grid, kSolveThreads, smem, s>>>(Q);
   GMG_CUDA(cudaGetLastError());
   return GMG_OK;
 }
