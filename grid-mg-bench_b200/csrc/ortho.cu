@@ -101,7 +101,11 @@ __device__ __forceinline__ bool block_active(const Params& P, int c) { return P.
 // one set of loads, the next KU steps' requests in flight meanwhile; the warps
 // split k and their sums are added in a fixed order.  32^4, 4^4 blocks, nbasis 32:
 // 2.49 ms (fragments by way of shared memory, 58 % of the pipe) -> 1.98 ms.
-template <int NT, bool CHECK>
+// HALF: the last tile holds four vectors at most, their real parts as rows 0 to 3 and
+// their imaginary parts as rows 4 to 7, so that it takes two MMAs against another tile and
+// one with itself instead of four and three (16^4, 4^4 blocks, nbasis 36: 282 -> 255 us;
+// the tiles of the real panel's Gram matrix before took 273).
+template <int NT, bool CHECK, bool HALF = false>
 __global__ void __launch_bounds__(NT > 4 ? 256 : 384) gram_kernel(Params P) {
   constexpr int KU = NT == 1 ? 8 : NT == 2 ? 4 : 2, NP = NT * (NT + 1) / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -112,7 +116,8 @@ __global__ void __launch_bounds__(NT > 4 ? 256 : 384) gram_kernel(Params P) {
   const int N = P.N, K = P.K, q = lane & 3;
   const double2* row[NT];  // rows past N read row N - 1: their sums are not used
 #pragma unroll
-  for (int X = 0; X < NT; ++X) row[X] = P.basis + ((int64_t)c * N + min(8 * X + (lane >> 2), N - 1)) * K;
+  for (int X = 0; X < NT; ++X)
+    row[X] = P.basis + ((int64_t)c * N + min(8 * X + (HALF && X == NT - 1 ? (lane >> 2) & 3 : lane >> 2), N - 1)) * K;
   double re[NP][2], im[NP][2];
 #pragma unroll
   for (int p = 0; p < NP; ++p) re[p][0] = re[p][1] = im[p][0] = im[p][1] = 0.0;
@@ -131,15 +136,26 @@ __global__ void __launch_bounds__(NT > 4 ? 256 : 384) gram_kernel(Params P) {
     if (u + nw < units) load(g, u + nw);
 #pragma unroll
     for (int t = 0; t < KU; ++t) {
+      constexpr int NW = HALF ? NT - 1 : NT;  // whole tiles
+      if constexpr (HALF) {
+        const double h = (lane >> 2) < 4 ? f[t][NW].x : f[t][NW].y;
+        constexpr int B = NW * (NW + 1) / 2;
 #pragma unroll
-      for (int X = 0; X < NT; ++X)
+        for (int Y = 0; Y < NW; ++Y) {
+          f64mma::mma(re[B + Y], h, f[t][Y].x);
+          f64mma::mma(im[B + Y], h, f[t][Y].y);
+        }
+        f64mma::mma(re[B + NW], h, h);
+      }
+#pragma unroll
+      for (int X = 0; X < NW; ++X)
 #pragma unroll
         for (int Y = 0; Y <= X; ++Y) {
           f64mma::mma(re[X * (X + 1) / 2 + Y], f[t][X].x, f[t][Y].x);
           f64mma::mma(im[X * (X + 1) / 2 + Y], f[t][X].x, f[t][Y].y);
         }
 #pragma unroll
-      for (int X = 0; X < NT; ++X)
+      for (int X = 0; X < NW; ++X)
 #pragma unroll
         for (int Y = 0; Y <= X; ++Y) {
           f64mma::mma(re[X * (X + 1) / 2 + Y], f[t][X].y, f[t][Y].y);
@@ -169,6 +185,11 @@ __global__ void __launch_bounds__(NT > 4 ? 256 : 384) gram_kernel(Params P) {
     const int at = (i & 7) * 8 + (j & 7), mirror = (j & 7) * 8 + (i & 7);
     double gr = 0.0, gi = 0.0;
     for (int v = 0; v < nw; ++v, d += NP * 128) {
+      if (HALF && X == NT - 1) {  // rows 0 to 3 and 4 to 7 (and columns, of the tile with itself)
+        gr += d[at] + (X == Y ? d[at + 36] : d[64 + at + 32]);
+        gi += (X == Y ? d[at + 4] : d[64 + at]) - d[at + 32];
+        continue;
+      }
       gr += d[at];
       gi += X == Y ? d[64 + at] - d[64 + mirror] : d[64 + at];
     }
@@ -653,12 +674,12 @@ static gmg_status workspace(gmg_agg* h, Params* P) {
   return GMG_OK;
 }
 
-template <int NT, bool CHECK>
+template <int NT, bool CHECK, bool HALF = false>
 static gmg_status launch_gram_nt(const Params& P, cudaStream_t s) {
   // four warps a block; eight where the blocks alone leave the chip's warps idle
   const int nw = P.Vc < num_sms() * 4 ? 8 : 4;
   const size_t smem = sizeof(double) * 128 * (NT * (NT + 1) / 2) * nw;
-  auto kern = gram_kernel<NT, CHECK>;
+  auto kern = gram_kernel<NT, CHECK, HALF>;
   GMG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<P.Vc, 32 * nw, smem, s>>>(P);
   GMG_CUDA(cudaGetLastError());
@@ -672,7 +693,10 @@ static gmg_status launch_gram(const Params& P, cudaStream_t s) {
     case 2: return launch_gram_nt<2, CHECK>(P, s);
     case 3: return launch_gram_nt<3, CHECK>(P, s);
     case 4: return launch_gram_nt<4, CHECK>(P, s);
-    case 5: return launch_gram_nt<5, CHECK>(P, s);
+    case 5:
+      if constexpr (!CHECK)
+        if (P.N <= 36) return launch_gram_nt<5, CHECK, true>(P, s);
+      return launch_gram_nt<5, CHECK>(P, s);
     default: return fail(GMG_ERR_UNSUPPORTED, "orthonormalise: nbasis above the tensor-core Gram path");
   }
 }
