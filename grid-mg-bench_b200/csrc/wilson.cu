@@ -471,9 +471,9 @@ __device__ __forceinline__ void wilson_site(const typename wt<T>::C* __restrict_
 // The backward hops read U_mu(x - mu) of the neighbour's run.  Per site and RHS
 // that is 1536 bytes in FP64, against 2112 for the site-major arrays, whose
 // 16-byte reads at 576- and 1152-byte strides also took a line each.  32^4, one
-// RHS: FP64 847 -> 380 to 420 us by machine (1.6 GB, 3.8 to 4.2 TB/s; where it takes
-// 380, 390 and 575 us at 4 and 5 CTAs per SM,
-// which spill), FP32 497 -> 168 us (189 at 4 CTAs per SM).
+// RHS: FP64 847 -> 380 to 420 us by machine (1.6 GB, 3.8 to 4.2 TB/s; 390 and 575 us at 4
+// and 5 CTAs per SM, which spill, where 3 take 380), FP32 497 -> 168 us (189 at 4 CTAs per
+// SM).
 constexpr int kSoa = 32, kSoaThreads = 128;
 
 template <class C>

@@ -141,7 +141,7 @@ def test_choices_by_kind_of_operator():
 
 
 def test_small_lattice_times_the_staged_kernel():
-    x = _field("f64", 12, 885, 256)
+    x = _field("f64", 24, 885, 256)  # 8.3 us staged, 18.5 us by tiles
     w = _handle(886, None, (4, 4, 4, 4))
     w.M(x, torch.zeros_like(x))
-    assert w.tuned_kernel("f64", 12) == "staged"
+    assert w.tuned_kernel("f64", 24) == "staged"
